@@ -54,9 +54,10 @@ __global__ void k_pow(const double* __restrict__ x, double* __restrict__ y, int6
     }
 }
 
-// Block-wide sum; result valid in thread 0.
+// Block-wide sum over T threads; result valid in thread 0.
+template <int T>
 __device__ __forceinline__ double block_sum(double v) {
-    __shared__ double warp_part[kOpThreads / 32];
+    __shared__ double warp_part[T / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
@@ -65,33 +66,98 @@ __device__ __forceinline__ double block_sum(double v) {
     __syncthreads();
     double r = 0.0;
     if (wid == 0) {
-        r = (lane < kOpThreads / 32) ? warp_part[lane] : 0.0;
+        r = (lane < T / 32) ? warp_part[lane] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
     }
     return r;
 }
 
-// mode 0: sum of squares, mode 1: plain sum.  Every CTA walks every segment with
-// a grid stride, so the partial of CTA b is a fixed function of the input: the
-// two-pass reduction is deterministic for a given grid.
+// Block-wide sum of an integer, valid in every thread (sizes of a block list).
+template <int T>
+__device__ __forceinline__ int64_t block_total(int64_t v) {
+    __shared__ int64_t part[T / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = v;
+    __syncthreads();
+    int64_t r = 0;
+#pragma unroll
+    for (int w = 0; w < T / 32; ++w) r += part[w];
+    return r;
+}
+
+__device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// mode 0: sum of squares, mode 1: plain sum.  Bound by HBM (8 bytes read per
+// coefficient).  The concatenated segments are cut into one contiguous share
+// per CTA, so that a CTA meets one or two segments whatever their number, and
+// each thread keeps eight 16-byte loads in flight (64 KB per CTA, two CTAs per
+// SM; the copy bandwidth needs about 40 KB per SM).  The share of CTA b is a
+// fixed function of the list, so the two-pass sum is deterministic.  12.2 M
+// coefficients in 9 segments: 76 us before (every CTA strode over every
+// segment, one 8-byte load per thread at a time), 17 us now.
+constexpr int kReduceThreads = 512;
+constexpr int kReduceUnroll = 8;
+
 template <int MODE>
-__global__ void __launch_bounds__(kOpThreads)
+__global__ void __launch_bounds__(kReduceThreads, 2)
     k_weighted_reduce(const double* __restrict__ x, const FsSegment* __restrict__ segs,
                       int64_t n_segs, double* __restrict__ partial) {
+    int64_t mine = 0;
+    for (int64_t s = threadIdx.x; s < n_segs; s += kReduceThreads) mine += segs[s].length;
+    const int64_t total = block_total<kReduceThreads>(mine);
+    int64_t share = ceil_div(total, gridDim.x);
+    if (share < kReduceThreads) share = kReduceThreads;
+    const int64_t begin = share * blockIdx.x;
+    const int64_t end = begin + share < total ? begin + share : total;
     double acc = 0.0;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t s = 0; s < n_segs; ++s) {
+    int64_t pos = 0;
+    for (int64_t s = 0; s < n_segs && pos < end; ++s) {
         const FsSegment sg = segs[s];
+        const int64_t lo = begin > pos ? begin - pos : 0;
+        const int64_t hi = end - pos < sg.length ? end - pos : sg.length;
+        pos += sg.length;
+        if (hi <= lo) continue;
+        const double* p = x + sg.offset + lo;
+        int64_t n = hi - lo;
         double part = 0.0;
-        for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-             i < sg.length; i += stride) {
-            const double v = __ldg(x + sg.offset + i);
+        // blocks start at any element: one leading element brings p to 16 bytes
+        if (reinterpret_cast<uintptr_t>(p) & 8) {
+            if (threadIdx.x == 0) part = (MODE == 0) ? p[0] * p[0] : p[0];
+            ++p;
+            --n;
+        }
+        const double2* p2 = reinterpret_cast<const double2*>(p);
+        const int64_t n2 = n / 2;
+        double sum[2] = {0.0, 0.0};
+        for (int64_t i = threadIdx.x; i < n2; i += kReduceThreads * kReduceUnroll) {
+            double2 v[kReduceUnroll];
+#pragma unroll
+            for (int u = 0; u < kReduceUnroll; ++u) {
+                const int64_t k = i + u * kReduceThreads;
+                v[u] = k < n2 ? __ldg(p2 + k) : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < kReduceUnroll; ++u) {
+                if (MODE == 0) {
+                    sum[0] = fma(v[u].x, v[u].x, sum[0]);
+                    sum[1] = fma(v[u].y, v[u].y, sum[1]);
+                } else {
+                    sum[0] += v[u].x;
+                    sum[1] += v[u].y;
+                }
+            }
+        }
+        if ((n & 1) && threadIdx.x == 1) {
+            const double v = __ldg(p + n - 1);
             part += (MODE == 0) ? v * v : v;
         }
+        part += sum[0] + sum[1];
         acc = fma(sg.weight, part, acc);
     }
-    const double r = block_sum(acc);
+    const double r = block_sum<kReduceThreads>(acc);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
@@ -99,56 +165,204 @@ __global__ void __launch_bounds__(kOpThreads)
     k_final_sum(const double* __restrict__ partial, int64_t n, double* __restrict__ out) {
     double acc = 0.0;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
-    const double r = block_sum(acc);
+    const double r = block_sum<kOpThreads>(acc);
     if (threadIdx.x == 0) out[0] = r;
 }
 
-__global__ void __launch_bounds__(kOpThreads)
+// Units of the block-list kernels below: kUnit consecutive elements where both
+// sides run in the same storage order, a kTile x kTile tile where they do not
+// (one side goes through shared memory, so that both are read or written in
+// rows of kTile consecutive doubles).  Units of all blocks are numbered block
+// by block; a CTA takes one contiguous range of them.  Rows of kTile + 1
+// doubles keep the transposed shared accesses free of bank conflicts.
+constexpr int kTile = 64;
+constexpr int kUnit = kTile * kTile;
+constexpr int kPerThread = kUnit / kOpThreads;   // 16
+constexpr int kRowStep = kOpThreads / 32;        // tile rows a pass covers
+
+// Pair: 0 trace, 1 same storage order (a plain dot product), 2 crossed.
+__device__ __forceinline__ int pair_kind(const FsPairBlock& p) {
+    return p.b_off < 0 ? 0 : (p.a_trans != 0) != (p.b_trans != 0) ? 1 : 2;
+}
+
+__device__ __forceinline__ int64_t pair_units(const FsPairBlock& p) {
+    const int64_t m = p.m, n = p.n;
+    switch (pair_kind(p)) {
+        case 0: return ceil_div(m < n ? m : n, kUnit);
+        case 1: return ceil_div(m * n, kUnit);
+        default: return ceil_div(m, kTile) * ceil_div(n, kTile);
+    }
+}
+
+// Bound by HBM (16 bytes read per coefficient pair).  The crossed form is the
+// usual one (two C-order blocks: A by rows, B by columns); with one element per
+// thread at a time B came in 8 useful bytes per 32-byte sector, after two
+// 64-bit divisions.  Here a thread issues its 32 loads of a tile pair before
+// the first use.  Two SU(2) corners of 13.1 M coefficients: 118 us before,
+// 37 us now.
+__global__ void __launch_bounds__(kOpThreads, 2)
     k_pair_contract(const double* __restrict__ a, const double* __restrict__ b,
                     const FsPairBlock* __restrict__ pairs, int64_t n_pairs,
                     double* __restrict__ partial) {
+    __shared__ double tile[kTile][kTile + 1];
+    int64_t mine = 0;
+    for (int64_t q = threadIdx.x; q < n_pairs; q += kOpThreads) mine += pair_units(pairs[q]);
+    const int64_t total = block_total<kOpThreads>(mine);
+    const int64_t begin = total * blockIdx.x / gridDim.x;
+    const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
+    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
     double acc = 0.0;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t q = 0; q < n_pairs; ++q) {
+    int64_t pos = 0;
+    for (int64_t q = 0; q < n_pairs && pos < end; ++q) {
         const FsPairBlock pb = pairs[q];
+        const int64_t units = pair_units(pb);
+        const int64_t lo = begin > pos ? begin - pos : 0;
+        const int64_t hi = end - pos < units ? end - pos : units;
+        pos += units;
+        const int kind = pair_kind(pb);
         double part = 0.0;
-        const int64_t m = pb.m, n = pb.n;
-        if (pb.b_off < 0) {  // trace
-            const int64_t d = m < n ? m : n;
-            for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-                 i < d; i += stride) {
-                part += __ldg(a + pb.a_off + (pb.a_trans ? i * m + i : i * n + i));
-            }
-        } else {
-            const int64_t total = m * n;
-            for (int64_t f = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-                 f < total; f += stride) {
-                const int64_t i = f / n, j = f % n;
-                const double av = __ldg(a + pb.a_off + (pb.a_trans ? j * m + i : f));
-                // B has logical shape (n, m); entry (j, i).
-                const double bv = __ldg(b + pb.b_off + (pb.b_trans ? i * n + j : j * m + i));
-                part = fma(av, bv, part);
+        const double* pa = a + pb.a_off;
+        const double* pbm = b + pb.b_off;
+        // storage of A: R rows of C (B then holds C rows of R)
+        const int64_t R = pb.a_trans ? pb.n : pb.m, C = pb.a_trans ? pb.m : pb.n;
+        for (int64_t u = lo; u < hi; ++u) {
+            if (kind == 0) {
+                const int64_t d = R < C ? R : C;
+#pragma unroll 4
+                for (int k = 0; k < kPerThread; ++k) {
+                    const int64_t i = u * kUnit + k * kOpThreads + threadIdx.x;
+                    if (i < d) part += __ldg(pa + i * C + i);
+                }
+            } else if (kind == 1) {
+                double va[kPerThread], vb[kPerThread];
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k) {
+                    const int64_t f = u * kUnit + k * kOpThreads + threadIdx.x;
+                    va[k] = f < R * C ? __ldg(pa + f) : 0.0;
+                    vb[k] = f < R * C ? __ldg(pbm + f) : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k) part = fma(va[k], vb[k], part);
+            } else {
+                const int64_t ct = ceil_div(C, kTile);
+                const int64_t r0 = (u / ct) * kTile, c0 = (u % ct) * kTile;
+                double va[kPerThread], vb[kPerThread];
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k) {
+                    const int i = wid + (k / 2) * kRowStep, j = lane + (k % 2) * 32;
+                    va[k] = (r0 + i < R && c0 + j < C) ? __ldg(pa + (r0 + i) * C + c0 + j) : 0.0;
+                    vb[k] = (c0 + i < C && r0 + j < R) ? __ldg(pbm + (c0 + i) * R + r0 + j) : 0.0;
+                }
+                __syncthreads();  // the previous tile has been read
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k)
+                    tile[wid + (k / 2) * kRowStep][lane + (k % 2) * 32] = vb[k];
+                __syncthreads();
+                // entries outside the block are zero in va only: B's zeros
+                // are placed at their own (c, r), inside the same mask
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k)
+                    part = fma(va[k], tile[lane + (k % 2) * 32][wid + (k / 2) * kRowStep], part);
             }
         }
         acc = fma(pb.weight, part, acc);
     }
-    const double r = block_sum(acc);
+    const double r = block_sum<kOpThreads>(acc);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
-__global__ void __launch_bounds__(kOpThreads)
+__device__ __forceinline__ int64_t diag_units(const FsDiagBlock& d) {
+    const int64_t m = d.m, n = d.n;
+    return d.x_trans ? ceil_div(m, kTile) * ceil_div(n, kTile) : ceil_div(m * n, kUnit);
+}
+
+// Bound by HBM (16 bytes per coefficient).  The row of an element comes from
+// one 32-bit multiply-high with the constants of the block's column count,
+// computed once per block, and a thread issues eight loads before its stores;
+// F-order inputs go through a shared tile.  12.2 M coefficients in 9 blocks:
+// 63 us before (a 64-bit division per element, one load at a time),
+// 36 us now.
+__global__ void __launch_bounds__(kOpThreads, 4)
     k_diag_mul(const double* __restrict__ x, const double* __restrict__ diag,
                double* __restrict__ out, const FsDiagBlock* __restrict__ blocks,
                int64_t n_blocks) {
-    for (int64_t q = blockIdx.y; q < n_blocks; q += gridDim.y) {
+    __shared__ double tile[kTile][kTile + 1];
+    int64_t mine = 0;
+    for (int64_t q = threadIdx.x; q < n_blocks; q += kOpThreads) mine += diag_units(blocks[q]);
+    const int64_t total = block_total<kOpThreads>(mine);
+    const int64_t begin = total * blockIdx.x / gridDim.x;
+    const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
+    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+    constexpr int kBatch = 8;
+    int64_t pos = 0;
+    for (int64_t q = 0; q < n_blocks && pos < end; ++q) {
         const FsDiagBlock db = blocks[q];
-        const int64_t m = db.m, n = db.n, total = m * n;
-        for (int64_t f = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-             f < total; f += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-            const int64_t i = f / n, j = f % n;
-            const double v = __ldg(x + db.x_off + (db.x_trans ? j * m + i : f));
-            const double d = __ldg(diag + db.d_off + (db.left ? i : j));
-            out[db.out_off + f] = v * d;
+        const int64_t units = diag_units(db);
+        const int64_t lo = begin > pos ? begin - pos : 0;
+        const int64_t hi = end - pos < units ? end - pos : units;
+        pos += units;
+        if (hi <= lo) continue;
+        const int64_t m = db.m, n = db.n;
+        const double* px = x + db.x_off;
+        const double* pd = diag + db.d_off;
+        double* po = out + db.out_off;
+        if (!db.x_trans) {
+            const uint32_t d = static_cast<uint32_t>(db.n);
+            const uint32_t sh = d > 1 ? 32 - __clz(d - 1) : 0;
+            const uint32_t mul = static_cast<uint32_t>(((((1ull << sh) - d) << 32) / d) + 1);
+            for (int64_t u = lo; u < hi; ++u) {
+                const int64_t f0 = u * kUnit;
+                const int64_t i0 = f0 / n;
+                const uint32_t j0 = static_cast<uint32_t>(f0 - i0 * n);
+                const int64_t left = m * n - f0;
+                const int cnt = left < kUnit ? static_cast<int>(left) : kUnit;
+#pragma unroll
+                for (int h = 0; h < kPerThread; h += kBatch) {
+                    double v[kBatch], w[kBatch];
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const int t = (h + k) * kOpThreads + threadIdx.x;
+                        v[k] = w[k] = 0.0;
+                        if (t < cnt) {
+                            v[k] = __ldg(px + f0 + t);
+                            const uint32_t l = j0 + t;
+                            const uint32_t r = fast_div(l, mul, sh);
+                            w[k] = __ldg(pd + (db.left ? i0 + r : static_cast<int64_t>(l - r * d)));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const int t = (h + k) * kOpThreads + threadIdx.x;
+                        if (t < cnt) po[f0 + t] = v[k] * w[k];
+                    }
+                }
+            }
+        } else {
+            const int64_t jt = ceil_div(n, kTile);
+            for (int64_t u = lo; u < hi; ++u) {
+                const int64_t i0 = (u / jt) * kTile, j0 = (u % jt) * kTile;
+                __syncthreads();  // the previous tile has been read
+#pragma unroll
+                for (int h = 0; h < kPerThread; h += kBatch) {
+                    double v[kBatch];
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const int j = wid + ((h + k) / 2) * kRowStep, i = lane + (k % 2) * 32;
+                        v[k] = (j0 + j < n && i0 + i < m) ? __ldg(px + (j0 + j) * m + i0 + i) : 0.0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k)
+                        tile[wid + ((h + k) / 2) * kRowStep][lane + (k % 2) * 32] = v[k];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k) {
+                    const int i = wid + (k / 2) * kRowStep, j = lane + (k % 2) * 32;
+                    if (i0 + i < m && j0 + j < n)
+                        po[(i0 + i) * n + j0 + j] =
+                            tile[j][i] * __ldg(pd + (db.left ? i0 + i : j0 + j));
+                }
+            }
         }
     }
 }
@@ -211,7 +425,7 @@ int weighted_reduce(const double* d_x, const FsSegment* d_segs, int64_t n_segs,
     if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
     if (n_segs > 0 && (d_x == nullptr || d_segs == nullptr)) return FS_ERR_INVALID_ARG;
     cudaStream_t s = fsb::as_stream(stream);
-    fsb::k_weighted_reduce<MODE><<<fsb::kReducePartials, fsb::kOpThreads, 0, s>>>(
+    fsb::k_weighted_reduce<MODE><<<fsb::kReducePartials, fsb::kReduceThreads, 0, s>>>(
         d_x, d_segs, n_segs, d_partial);
     int st = fsb::launch_status();
     if (st != FS_OK) return st;
@@ -254,8 +468,8 @@ extern "C" int fs_diag_mul(const double* d_x, const double* d_diag, double* d_ou
     if (n_blocks == 0) return FS_OK;
     if (d_x == nullptr || d_diag == nullptr || d_out == nullptr || d_blocks == nullptr)
         return FS_ERR_INVALID_ARG;
-    dim3 grid(fsb::num_sms(), static_cast<unsigned>(n_blocks < 65535 ? n_blocks : 65535));
-    fsb::k_diag_mul<<<grid, fsb::kOpThreads, 0, fsb::as_stream(stream)>>>(d_x, d_diag, d_out,
-                                                                          d_blocks, n_blocks);
+    // one wave of resident CTAs; CTAs without a unit return at once
+    fsb::k_diag_mul<<<4 * fsb::num_sms(), fsb::kOpThreads, 0, fsb::as_stream(stream)>>>(
+        d_x, d_diag, d_out, d_blocks, n_blocks);
     return fsb::launch_status();
 }
