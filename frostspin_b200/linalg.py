@@ -119,40 +119,71 @@ def shared_launches():
         _SHARED = old
 
 
-def defer_permute(ebs, tasks, src, out, nbytes):
-    """Queue one abelian permute (its host EB and task tables, source and
-    destination buffers) for the enclosing shared_launches block; returns
-    False when no block is open."""
+def upload_copies(tables):
+    """Device copies of the tables of a batch of strided copies: the EBs, the row
+    tasks of fs_abelian_permute and the tile tasks of fs_permute_tiles (None
+    when no EB is transposed)."""
+    ebs, tasks, tiles = tables
+    return dev.upload(ebs), dev.upload(tasks), dev.upload(tiles) if tiles.size else None
+
+
+def run_copies(tables, device_tables, src, out):
+    """One batch of strided copies src -> out: the row tasks in one launch, the
+    transposed ones, if any, in another."""
+    ebs, tasks, tiles = tables
+    d_ebs, d_tasks, d_tiles = device_tables
+    if tasks.size or d_tiles is None:
+        _native.call("fs_abelian_permute", dev.ptr(src), src.numel(), dev.ptr(out), out.numel(),
+                     d_ebs.data_ptr(), ebs.size, d_tasks.data_ptr(), tasks.size, None,
+                     dev.stream())
+    if d_tiles is not None:
+        _native.call("fs_permute_tiles", dev.ptr(src), src.numel(), dev.ptr(out), out.numel(),
+                     d_ebs.data_ptr(), ebs.size, d_tiles.data_ptr(), tiles.size, None,
+                     dev.stream())
+
+
+def defer_permute(tables, src, out, nbytes):
+    """Queue one abelian permute (its host tables, source and destination
+    buffers) for the enclosing shared_launches block; returns False when no
+    block is open."""
     if _SHARED is None:
         return False
-    _SHARED["perm"].append((ebs, tasks, src, out, nbytes))
+    _SHARED["perm"].append((tables, src, out, nbytes))
     return True
 
 
 def _flush_permutes(items):
     bufs = np.zeros(len(items), dtype=_native.PERM_BUFFERS_DTYPE)
-    ebs_all, tasks_all = [], []
+    ebs_all, tasks_all, tiles_all = [], [], []
     n_eb = 0
     nbytes = 0.0
-    for i, (ebs, tasks, src, out, nb) in enumerate(items):
+    for i, ((ebs, tasks, tiles), src, out, nb) in enumerate(items):
         bufs[i] = (dev.ptr(src), int(src.numel()), dev.ptr(out), int(out.numel()))
         e = ebs.copy()
         e["pad"] = i
-        t = tasks.copy()
-        t["eb"] += n_eb
+        for table, every in ((tasks, tasks_all), (tiles, tiles_all)):
+            t = table.copy()
+            t["eb"] += n_eb
+            every.append(t)
         n_eb += e.size
         ebs_all.append(e)
-        tasks_all.append(t)
         nbytes += nb
     ebs_all = np.concatenate(ebs_all)
     tasks_all = np.concatenate(tasks_all)
-    if tasks_all.size == 0:
+    tiles_all = np.concatenate(tiles_all)
+    if ebs_all.size == 0:
         return
-    d_bufs, d_ebs, d_tasks = dev.upload(bufs), dev.upload(ebs_all), dev.upload(tasks_all)
+    d_bufs = dev.upload(bufs)
+    d_ebs, d_tasks, d_tiles = upload_copies((ebs_all, tasks_all, tiles_all))
     with instrument.region("permute", bytes=nbytes):
-        _native.call("fs_abelian_permute_multi", d_bufs.data_ptr(), bufs.size,
-                     d_ebs.data_ptr(), ebs_all.size, d_tasks.data_ptr(), tasks_all.size,
-                     None, dev.stream())
+        if tasks_all.size or d_tiles is None:
+            _native.call("fs_abelian_permute_multi", d_bufs.data_ptr(), bufs.size,
+                         d_ebs.data_ptr(), ebs_all.size, d_tasks.data_ptr(), tasks_all.size,
+                         None, dev.stream())
+        if d_tiles is not None:
+            _native.call("fs_permute_tiles_multi", d_bufs.data_ptr(), bufs.size,
+                         d_ebs.data_ptr(), ebs_all.size, d_tiles.data_ptr(), tiles_all.size,
+                         None, dev.stream())
 
 
 @contextlib.contextmanager

@@ -150,6 +150,7 @@ class AbelianPermutePlan:
         "size",
         "ebs",
         "tasks",
+        "tiles",
         "in_len",
         "device_tables",
     )
@@ -309,6 +310,7 @@ def build_abelian_permute_plan(
     plan.size = total
     plan.ebs = ebs
     plan.tasks = _make_tasks(ebs)
+    plan.tiles = _make_tile_tasks(ebs)
     plan.in_len = int(in_len)
     plan.device_tables = None
     return plan
@@ -372,15 +374,54 @@ def _pack_ebs(dims, ostride, nstride, obase, nbase, present):
     m, s = magic_divisor(out["dims"])
     out["divm"] = m
     out["divs"] = s
+    _choose_tile_legs(out, r, present)
     return out, vol
 
 
+def _choose_tile_legs(ebs, r, present):
+    """Set tile_leg where the source runs along another leg than the output."""
+    rows = np.arange(ebs.size)
+    last = r - 1
+    unit = (
+        (ebs["ostride"] == 1)
+        & (np.arange(FS_PERM_MAXR) < last[:, None])
+        & (ebs["dims"] >= TILE_MIN)
+    )
+    ok = (
+        np.asarray(present, dtype=bool)
+        & unit.any(axis=1)
+        & (ebs["ostride"][rows, last] != 1)
+        & (ebs["nstride"][rows, last] == 1)
+        & (ebs["dims"][rows, last] >= TILE_MIN)
+    )
+    leg = unit.argmax(axis=1)
+    area = ebs["dims"][rows, leg].astype(np.int64) * ebs["dims"][rows, last]
+    ok &= area >= TILE_AREA
+    if int(ebs["volume"][ok].astype(np.int64).sum()) >= TILE_TOTAL:
+        ebs["tile_leg"] = np.where(ok, leg, -1)
+
+
 MAX_TASK_ROWS = 1024
+TILE = 32             # edge of a transposed tile (kTileEdge)
+# EBs that run in tiles: both legs at least 6 long and at least 128 entries in
+# their plane.  8 M coefficients, rows against tiles: legs 6 x 40 55 / 45 us,
+# 12 x 12 56 / 42 us, 100 x 6 52 / 47 us, 24 x 24 58 / 29 us; but 8 x 8 60 / 68
+# us and 4 x 4 55 / 221 us, where a warp's 32 lanes are mostly idle.
+TILE_MIN = 6
+TILE_AREA = 128
+# ... and at least this many entries in all such EBs of a permute: below it the
+# tensor stays in L2, where rows cost no DRAM sectors, and the tiles are a second
+# launch (edge tensors of 0.28 M entries 6.1 us by rows, 7.1 by tiles; 1.1 M 9.0
+# and 10.5; 2.5 M 17.5 and 12.2; 4.5 M 29.6 and 17.8).
+TILE_TOTAL = 1_500_000
+MAX_TASK_TILES = 32   # kTileTaskMax
+TILE_TASKS = 4 * 3 * 148 * 4   # four tasks for every resident warp of the tile kernel
 
 
 def _make_tasks(ebs, chunk=TASK_CHUNK):
-    """Split every EB into tasks of whole rows (runs along the last leg): about
-    `chunk` entries and at most MAX_TASK_ROWS rows per task."""
+    """Split every EB without a tile_leg into tasks of whole rows (runs along
+    the last leg): about `chunk` entries and at most MAX_TASK_ROWS rows per
+    task."""
     n_eb = ebs.size
     if n_eb == 0:
         return np.zeros(0, dtype=PERM_TASK_DTYPE)
@@ -388,15 +429,34 @@ def _make_tasks(ebs, chunk=TASK_CHUNK):
     inner = ebs["dims"][np.arange(n_eb), r - 1].astype(np.int64)
     rows = ebs["volume"].astype(np.int64) // inner
     per = np.clip(chunk // inner, 1, MAX_TASK_ROWS)
-    nchunk = (rows + per - 1) // per
+    return _cut(np.where(ebs["tile_leg"] < 0, rows, 0), per)
+
+
+def _make_tile_tasks(ebs):
+    """Tasks of the EBs with a tile_leg: ranges of their tiles (outer legs, then
+    tiles along the last leg, then along tile_leg), sized for a few tasks per
+    resident warp."""
+    leg = ebs["tile_leg"].astype(np.int64)
+    i = np.arange(ebs.size)
+    da = ebs["dims"][i, leg].astype(np.int64)
+    db = ebs["dims"][i, ebs["ndim"].astype(np.int64) - 1].astype(np.int64)
+    outer = ebs["volume"].astype(np.int64) // np.maximum(da * db, 1)
+    units = np.where(leg >= 0, outer * -(-da // TILE) * -(-db // TILE), 0)
+    per = np.clip(int(units.sum()) // TILE_TASKS, 1, MAX_TASK_TILES)
+    return _cut(units, np.full(ebs.size, per))
+
+
+def _cut(units, per):
+    """FsPermTask table cutting units[e] units of every EB e into runs of per[e]."""
+    nchunk = (units + per - 1) // per
     n = int(nchunk.sum())
     tasks = np.zeros(n, dtype=PERM_TASK_DTYPE)
-    eb = np.repeat(np.arange(n_eb), nchunk)
+    eb = np.repeat(np.arange(units.size), nchunk)
     first = np.repeat(np.cumsum(nchunk) - nchunk, nchunk)
     start = (np.arange(n) - first) * per[eb]
     tasks["eb"] = eb
     tasks["start"] = start
-    tasks["count"] = np.minimum(per[eb], rows[eb] - start)
+    tasks["count"] = np.minimum(per[eb], units[eb] - start)
     return tasks
 
 

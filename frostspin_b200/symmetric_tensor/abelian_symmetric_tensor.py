@@ -11,7 +11,7 @@ from collections import OrderedDict
 import numpy as np
 import torch
 
-from .. import _native, instrument, linalg
+from .. import instrument, linalg
 from .. import device as dev
 from .abelian_plan import (
     GroupInfo,
@@ -183,25 +183,12 @@ class AbelianSymmetricTensor(SymmetricTensor):
         """abelian_symmetric_tensor.py:395-430 on the device."""
         plan = self._permute_plan(axes, nrr)
         out = dev.empty_f64(plan.size)
-        if plan.size and linalg.defer_permute(plan.ebs, plan.tasks, self._data, out,
-                                              16.0 * plan.size):
+        tables = (plan.ebs, plan.tasks, plan.tiles)
+        if plan.size and linalg.defer_permute(tables, self._data, out, 16.0 * plan.size):
             return out, plan.offsets, plan.block_shapes, plan.block_irreps
         if plan.size:
             if plan.device_tables is None:
-                plan.device_tables = (dev.upload(plan.ebs), dev.upload(plan.tasks))
-            d_ebs, d_tasks = plan.device_tables
+                plan.device_tables = linalg.upload_copies(tables)
             with instrument.region("permute", bytes=16.0 * plan.size):
-                _native.call(
-                    "fs_abelian_permute",
-                    dev.ptr(self._data),
-                    int(self._data.numel()),
-                    dev.ptr(out),
-                    int(out.numel()),
-                    d_ebs.data_ptr(),
-                    int(plan.ebs.size),
-                    d_tasks.data_ptr(),
-                    int(plan.tasks.size),
-                    None,
-                    dev.stream(),
-                )
+                linalg.run_copies(tables, plan.device_tables, self._data, out)
         return out, plan.offsets, plan.block_shapes, plan.block_irreps

@@ -4,9 +4,9 @@ two-leg elementary block per irrep block."""
 
 import numpy as np
 
-from .. import _native
 from .. import device as dev
-from .abelian_plan import _make_tasks, _pack_ebs
+from .. import linalg
+from .abelian_plan import _make_tasks, _make_tile_tasks, _pack_ebs
 
 
 def relayout_blocks(data, offsets, shapes, trans, new_offsets, total):
@@ -26,20 +26,6 @@ def relayout_blocks(data, offsets, shapes, trans, new_offsets, total):
     present = np.ones(nb, dtype=bool)
     ebs, vol = _pack_ebs(dims, ostride, nstride, np.asarray(offsets, dtype=np.int64),
                          np.asarray(new_offsets, dtype=np.int64), present)
-    tasks = _make_tasks(ebs)
-    d_ebs = dev.upload(ebs)
-    d_tasks = dev.upload(tasks)
-    _native.call(
-        "fs_abelian_permute",
-        dev.ptr(data),
-        data.numel(),
-        dev.ptr(out),
-        out.numel(),
-        d_ebs.data_ptr(),
-        ebs.size,
-        d_tasks.data_ptr(),
-        tasks.size,
-        None,
-        dev.stream(),
-    )
+    tables = (ebs, _make_tasks(ebs), _make_tile_tasks(ebs))
+    linalg.run_copies(tables, linalg.upload_copies(tables), data, out)
     return out

@@ -36,7 +36,7 @@ from .. import _native, instrument, linalg
 from .. import device as dev
 from .._native import FS_PERM_MAXR
 from . import su2_fused_plan
-from .abelian_plan import _make_tasks, _pack_ebs
+from .abelian_plan import _make_tasks, _make_tile_tasks, _pack_ebs
 from .symmetric_tensor import SymmetricTensor
 
 _MAP_CACHE = OrderedDict()
@@ -149,7 +149,7 @@ def _copy_tables(dims, ostride, nstride, obase, nbase, present, src_len, dst_len
         dims, ostride, nstride, np.where(present, obase, -1), nbase, present
     )
     ebs, _ = _pack_ebs(dims, ostride, nstride, np.where(present, obase, -1), nbase, present)
-    return ebs, _make_tasks(ebs)
+    return ebs, _make_tasks(ebs), _make_tile_tasks(ebs)
 
 
 class LieMap:
@@ -166,12 +166,11 @@ class LieMap:
         if self.device is None:
             fz = self.fused
             self.device = (
-                dev.upload(self.gather[0]), dev.upload(self.gather[1]),
-                dev.upload(self.scatter[0]), dev.upload(self.scatter[1]),
+                linalg.upload_copies(self.gather), linalg.upload_copies(self.scatter),
                 dev.upload_f64(self.u_host),
                 None if fz is None else tuple(dev.upload(a) for a in fz),
             )
-        g_ebs, g_tasks, s_ebs, s_tasks, d_u, d_fz = self.device
+        d_gather, d_scatter, d_u, d_fz = self.device
         if out is None:
             out = dev.zeros_f64(self.out_size) if self.zero_out else dev.empty_f64(self.out_size)
         if src.numel() < self.in_len:
@@ -191,11 +190,7 @@ class LieMap:
         x = dev.empty_f64(self.x_size)
         y = dev.empty_f64(int((self.M * self.N).sum()))
         with instrument.region("permute", bytes=16.0 * self.x_size):
-            _native.call(
-                "fs_abelian_permute", dev.ptr(src), int(src.numel()), dev.ptr(x),
-                int(x.numel()), g_ebs.data_ptr(), int(self.gather[0].size),
-                g_tasks.data_ptr(), int(self.gather[1].size), None, dev.stream(),
-            )
+            linalg.run_copies(self.gather, d_gather, src, x)
         arr = np.zeros(self.M.size, dtype=_native.GEMM_PROBLEM_DTYPE)
         y_off = _exclusive_cumsum(self.M * self.N)
         arr["A"] = d_u.data_ptr() + 8 * self.u_off
@@ -208,11 +203,7 @@ class LieMap:
         arr["alpha"] = 1.0
         linalg.grouped_dgemm_table(arr, region="gemm_recoupling")
         with instrument.region("permute", bytes=16.0 * int(y.numel())):
-            _native.call(
-                "fs_abelian_permute", dev.ptr(y), int(y.numel()), dev.ptr(out),
-                int(out.numel()), s_ebs.data_ptr(), int(self.scatter[0].size),
-                s_tasks.data_ptr(), int(self.scatter[1].size), None, dev.stream(),
-            )
+            linalg.run_copies(self.scatter, d_scatter, y, out)
         return out
 
 

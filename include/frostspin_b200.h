@@ -106,6 +106,20 @@ int fs_abelian_permute(const double* d_in, int64_t in_len, double* d_out,
                        const FsPermTask* d_tasks, int64_t n_tasks,
                        int32_t* d_flag, void* stream);
 
+/*
+ * The same copies for EBs whose unit-stride input leg is not the
+ * output-innermost one: tile_leg names it (ostride[tile_leg] == 1, and
+ * nstride == 1 on the last leg).  Tasks number 32 x 32 tiles of these two legs
+ * (outer legs, then tiles along the last leg, then along tile_leg), at most 32
+ * per task.  A permute is the row tasks of the EBs with tile_leg < 0 through
+ * fs_abelian_permute and the tile tasks of the others through this call, in
+ * either order.  fs_permute_tiles_multi: EB e uses the buffers bufs[e.pad].
+ */
+int fs_permute_tiles(const double* d_in, int64_t in_len, double* d_out,
+                     int64_t out_len, const FsPermEB* d_ebs, int64_t n_ebs,
+                     const FsPermTask* d_tasks, int64_t n_tasks,
+                     int32_t* d_flag, void* stream);
+
 /* -------------------------------------------------- fused SU(2) permute */
 /*
  * Replaces LieGroupSymmetricTensor._lie_permute_data -> fill_blocks_out ->
@@ -177,6 +191,10 @@ typedef struct FsPermBuffers {
 int fs_abelian_permute_multi(const FsPermBuffers* d_bufs, int64_t n_bufs,
                              const FsPermEB* d_ebs, int64_t n_ebs, const FsPermTask* d_tasks,
                              int64_t n_tasks, int32_t* d_flag, void* stream);
+int fs_permute_tiles_multi(const FsPermBuffers* d_bufs, int64_t n_bufs,
+                           const FsPermEB* d_ebs, int64_t n_ebs,
+                           const FsPermTask* d_tasks, int64_t n_tasks,
+                           int32_t* d_flag, void* stream);
 
 /* ------------------------------------------------------- grouped FP64 GEMM */
 /*
