@@ -19,8 +19,15 @@ from .._native import FS_PERM_MAXR, PERM_TASK_DTYPE, SU2_GROUP_DTYPE, SU2_PIECE_
 from .abelian_plan import magic_divisor
 
 MAXD = 8
-TASK_COLUMNS = 4096
-TASK_ROWS = 48      # FS_SU2_TASK_ROWS: outer-leg values one task may span
+TASK_TABLE = 1536   # FS_SU2_TASK_TABLE: (piece, row) offsets one task may hold
+TASK_ROWS = 768    # outer-leg values of a task of two pieces
+# Input coefficients of a task: enough to hide its descriptors behind the data
+# (TASK_COEFFS), fewer when the whole permute has less than one such task per
+# resident CTA (4 on each of 148 SMs)
+TASK_COEFFS = 16384
+TASK_COLUMNS = TASK_COEFFS   # longest task, a group with one row
+TASK_COEFFS_MIN = 2048
+TASKS = 4 * 148
 
 
 def fusable(M, K, E, e_out, n_in, n_out, max_rows, max_pieces):
@@ -139,33 +146,35 @@ def check(gtab, pieces, src_len, out_len, u_len):
 
 def make_tasks(gtab):
     """Tasks of the fused kernel: whole rows of the innermost output leg (L
-    columns each), at most TASK_ROWS rows and about TASK_COLUMNS columns per
-    task; a row longer than TASK_COLUMNS is cut into pieces of one row."""
-    ng = gtab.size
+    columns each) up to the task's coefficients and the rows its offset table
+    holds; a longer row is cut into pieces of one row.  Largest first, for the
+    kernel's static schedule."""
     ncols = gtab["ncols"].astype(np.int64)
     nd = gtab["ndim"].astype(np.int64)
-    L = np.where(nd > 0, gtab["dims"][np.arange(ng), np.maximum(nd - 1, 0)], 1).astype(np.int64)
-    per = np.where(L >= TASK_COLUMNS, TASK_COLUMNS,
-                   L * np.clip(TASK_COLUMNS // np.maximum(L, 1), 1, TASK_ROWS))
-    starts, groups_of = [], []
-    for g in range(ng):
-        if L[g] >= TASK_COLUMNS:
-            rows = np.arange(0, ncols[g], L[g])
-            inner = np.arange(0, L[g], TASK_COLUMNS)
-            st = (rows[:, None] + inner[None, :]).ravel()
-        else:
-            st = np.arange(0, ncols[g], per[g])
-        starts.append(st)
-        groups_of.append(np.full(st.size, g))
-    tasks = np.zeros(int(sum(x.size for x in starts)), dtype=PERM_TASK_DTYPE)
-    if tasks.size == 0:
-        return tasks
-    st = np.concatenate(starts)
-    gi = np.concatenate(groups_of)
-    tasks["eb"] = gi
-    tasks["start"] = st
-    row_end = np.where(L[gi] >= TASK_COLUMNS, (st // L[gi] + 1) * L[gi], ncols[gi])
-    tasks["count"] = np.minimum(np.minimum(per[gi], row_end - st), ncols[gi] - st)
+    i = np.arange(gtab.size)
+    L = np.maximum(np.where(nd > 0, gtab["dims"][i, np.maximum(nd - 1, 0)], 1).astype(np.int64), 1)
+    K = np.maximum(gtab["K"].astype(np.int64), 1)
+    pieces = gtab["in_count"].astype(np.int64) + gtab["out_count"]
+    rows = np.minimum(TASK_TABLE // np.maximum(pieces, 2), TASK_ROWS)
+    coeffs = np.clip(int((ncols * K).sum()) // TASKS, TASK_COEFFS_MIN, TASK_COEFFS)
+    cols = np.maximum(coeffs // K, 1)
+    # a unit is a run of whole rows, or a part of one row
+    whole = L <= cols
+    per = np.where(whole, L * np.clip(cols // L, 1, rows), cols)
+    line = np.where(whole, ncols, np.minimum(L, ncols))     # units do not cross lines
+    chunks = -(-line // np.maximum(per, 1))
+    count = chunks * np.where(whole, 1, -(-ncols // np.maximum(line, 1)))
+    g = np.repeat(i, count)
+    k = np.arange(int(count.sum())) - np.repeat(np.cumsum(count) - count, count)
+    row, part = k // chunks[g], k % chunks[g]
+    start = row * line[g] + part * per[g]
+    end = np.minimum((row + 1) * line[g], ncols[g])
+    size = np.minimum(per[g], end - start)
+    order = np.argsort(-size * K[g], kind="stable")
+    tasks = np.zeros(g.size, dtype=PERM_TASK_DTYPE)
+    tasks["eb"] = g[order]
+    tasks["start"] = start[order]
+    tasks["count"] = size[order]
     return tasks
 
 

@@ -138,13 +138,15 @@ int fs_permute_tiles(const double* d_in, int64_t in_len, double* d_out,
  * in_first .. in_first + in_count - 1 are the group's inputs, out_first .. its
  * outputs.  Tasks are FsPermTask with eb = group index, start = first column,
  * count = number of columns; the columns of a task span at most
- * FS_SU2_TASK_ROWS values of the outer legs (all legs but the innermost), a
- * task that spans more is skipped and flagged.  Limits: fs_su2_fused_limits.
+ * max(FS_SU2_TASK_ROWS, FS_SU2_TASK_TABLE / (in_count + out_count)) values of
+ * the outer legs (all legs but the innermost), a task that spans more is
+ * skipped and flagged.  Limits: fs_su2_fused_limits.
  * Accesses outside a buffer are skipped and raise FS_ERR_BOUNDS in *d_flag (if
  * not null).
  */
 #define FS_SU2_MAXD 8
 #define FS_SU2_TASK_ROWS 48
+#define FS_SU2_TASK_TABLE 1536   /* 32 pieces of FS_SU2_TASK_ROWS rows */
 
 typedef struct FsSu2Group {
     int64_t u_off;
