@@ -44,6 +44,12 @@ PERM_TASK_DTYPE = np.dtype(
 
 FS_SU2_MAXD = 8
 
+# host tables passed by value with a launch
+FS_LIST_MAX = 96
+FS_DGEMM_LIST_MAX = 360
+FS_SPLIT_LIST_MAX = 48
+FS_DGEMM_TILES, FS_DGEMM_UNIFORM, FS_DGEMM_THIN = range(3)
+
 SU2_GROUP_DTYPE = np.dtype(
     [
         ("u_off", "<i8"),
@@ -272,7 +278,9 @@ SIGNATURES = {
     "fs_thin_dgemm_shape": (ctypes.c_int, [_P, _P, _P]),
     "fs_grouped_dgemm_thin": (ctypes.c_int, [_P, _I64, _P, _I64, _P]),
     "fs_grouped_dgemm_uniform": (ctypes.c_int, [_P, _I64, _P, _I64, _I32, _I32, _P]),
+    "fs_grouped_dgemm_list": (ctypes.c_int, [_P, _I64, _I32, _P]),
     "fs_splitk_reduce": (ctypes.c_int, [_P, _I64, _I64, _P]),
+    "fs_splitk_reduce_list": (ctypes.c_int, [_P, _I64, _I64, _P]),
     "fs_expand_tiles": (ctypes.c_int, [_P, _I64, _I64, _P, _P]),
     "fs_ozaki_geometry": (ctypes.c_int, [_P, _P, _P, _P]),
     "fs_ozaki_split": (ctypes.c_int, [_P, _I64, _I32, _I32, _I32, _P]),
@@ -293,8 +301,11 @@ SIGNATURES = {
     "fs_reduce_partials": (ctypes.c_int, []),
     "fs_weighted_sumsq": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
     "fs_weighted_sum": (ctypes.c_int, [_P, _P, _I64, _P, _I64, _P, _P]),
+    "fs_weighted_sum_list": (ctypes.c_int, [_P, _P, _I64, _I32, _P, _I64, _P, _P]),
     "fs_pair_contract": (ctypes.c_int, [_P, _P, _P, _I64, _P, _I64, _P, _P]),
+    "fs_pair_contract_list": (ctypes.c_int, [_P, _P, _P, _I64, _P, _I64, _P, _P]),
     "fs_diag_mul": (ctypes.c_int, [_P, _P, _P, _P, _I64, _P]),
+    "fs_diag_mul_list": (ctypes.c_int, [_P, _P, _P, _P, _I64, _P]),
     "fs_o2_recombine": (ctypes.c_int, [_P, _I64, _P, _I64, _P, _I64, _P, _P, _I64, _P, _P]),
 }
 
@@ -351,10 +362,13 @@ def kernel_launches():
     return sum(LAUNCHES_PER_CALL.get(k, 0) * v for k, v in CALL_COUNTS.items())
 
 
-def call(name, *args):
-    """Call a C ABI function by name and raise on a non-zero status."""
-    st = getattr(lib(), name)(*args)
-    check(st, name)
+def call(name, *args, entry=None):
+    """Call a C ABI function by name and raise on a non-zero status.  `entry`: the
+    function to call when it is another form of `name` (the same kernel with its
+    table passed by value); the call counts as `name`."""
+    st = getattr(lib(), entry or name)(*args)
+    if st != FS_OK:
+        check(st, entry or name)
     CALL_COUNTS[name] = CALL_COUNTS.get(name, 0) + 1
     return st
 

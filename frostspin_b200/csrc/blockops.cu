@@ -101,9 +101,9 @@ __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 constexpr int kReduceThreads = 512;
 constexpr int kReduceUnroll = 8;
 
-template <int MODE>
+template <int MODE, class Table>
 __global__ void __launch_bounds__(kReduceThreads, 2)
-    k_weighted_reduce(const double* __restrict__ x, const FsSegment* __restrict__ segs,
+    k_weighted_reduce(const double* __restrict__ x, const __grid_constant__ Table segs,
                       int64_t n_segs, double* __restrict__ partial) {
     int64_t mine = 0;
     for (int64_t s = threadIdx.x; s < n_segs; s += kReduceThreads) mine += segs[s].length;
@@ -200,9 +200,10 @@ __device__ __forceinline__ int64_t pair_units(const FsPairBlock& p) {
 // 64-bit divisions.  Here a thread issues its 32 loads of a tile pair before
 // the first use.  Two SU(2) corners of 13.1 M coefficients: 118 us before,
 // 37 us now.
+template <class Table>
 __global__ void __launch_bounds__(kOpThreads, 2)
     k_pair_contract(const double* __restrict__ a, const double* __restrict__ b,
-                    const FsPairBlock* __restrict__ pairs, int64_t n_pairs,
+                    const __grid_constant__ Table pairs, int64_t n_pairs,
                     double* __restrict__ partial) {
     __shared__ double tile[kTile][kTile + 1];
     int64_t mine = 0;
@@ -282,9 +283,10 @@ __device__ __forceinline__ int64_t diag_units(const FsDiagBlock& d) {
 // F-order inputs go through a shared tile.  12.2 M coefficients in 9 blocks:
 // 63 us before (a 64-bit division per element, one load at a time),
 // 36 us now.
+template <class Table>
 __global__ void __launch_bounds__(kOpThreads, 4)
     k_diag_mul(const double* __restrict__ x, const double* __restrict__ diag,
-               double* __restrict__ out, const FsDiagBlock* __restrict__ blocks,
+               double* __restrict__ out, const __grid_constant__ Table blocks,
                int64_t n_blocks) {
     __shared__ double tile[kTile][kTile + 1];
     int64_t mine = 0;
@@ -418,58 +420,119 @@ extern "C" int fs_pow(const double* d_x, double* d_y, int64_t n, double p, void*
 }
 
 namespace {
-template <int MODE>
-int weighted_reduce(const double* d_x, const FsSegment* d_segs, int64_t n_segs,
-                    double* d_partial, int64_t n_partial, double* d_out, void* stream) {
-    if (n_segs < 0 || n_partial < fsb::kReducePartials) return FS_ERR_INVALID_ARG;
+
+template <int MODE, class Table>
+int weighted_reduce(const double* d_x, const Table& segs, int64_t n_segs, double* d_partial,
+                    int64_t n_partial, double* d_out, void* stream) {
+    if (n_partial < fsb::kReducePartials) return FS_ERR_INVALID_ARG;
     if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
-    if (n_segs > 0 && (d_x == nullptr || d_segs == nullptr)) return FS_ERR_INVALID_ARG;
+    if (n_segs > 0 && d_x == nullptr) return FS_ERR_INVALID_ARG;
     cudaStream_t s = fsb::as_stream(stream);
     fsb::k_weighted_reduce<MODE><<<fsb::kReducePartials, fsb::kReduceThreads, 0, s>>>(
-        d_x, d_segs, n_segs, d_partial);
+        d_x, segs, n_segs, d_partial);
     int st = fsb::launch_status();
     if (st != FS_OK) return st;
     fsb::k_final_sum<<<1, fsb::kOpThreads, 0, s>>>(d_partial, fsb::kReducePartials, d_out);
     return fsb::launch_status();
 }
+
+template <class Table>
+int pair_contract(const double* d_a, const double* d_b, const Table& pairs, int64_t n_pairs,
+                  double* d_partial, int64_t n_partial, double* d_out, void* stream) {
+    if (n_partial < fsb::kReducePartials) return FS_ERR_INVALID_ARG;
+    if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
+    if (n_pairs > 0 && d_a == nullptr) return FS_ERR_INVALID_ARG;
+    cudaStream_t s = fsb::as_stream(stream);
+    fsb::k_pair_contract<<<fsb::kReducePartials, fsb::kOpThreads, 0, s>>>(d_a, d_b, pairs, n_pairs,
+                                                                          d_partial);
+    int st = fsb::launch_status();
+    if (st != FS_OK) return st;
+    fsb::k_final_sum<<<1, fsb::kOpThreads, 0, s>>>(d_partial, fsb::kReducePartials, d_out);
+    return fsb::launch_status();
+}
+
+template <class Table>
+int diag_mul(const double* d_x, const double* d_diag, double* d_out, const Table& blocks,
+             int64_t n_blocks, void* stream) {
+    if (d_x == nullptr || d_diag == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
+    // one wave of resident CTAs; CTAs without a unit return at once
+    fsb::k_diag_mul<<<4 * fsb::num_sms(), fsb::kOpThreads, 0, fsb::as_stream(stream)>>>(
+        d_x, d_diag, d_out, blocks, n_blocks);
+    return fsb::launch_status();
+}
+
+using SegmentList = fsb::InlineTable<FsSegment, FS_LIST_MAX>;
+using PairList = fsb::InlineTable<FsPairBlock, FS_LIST_MAX>;
+using DiagList = fsb::InlineTable<FsDiagBlock, FS_LIST_MAX>;
+static_assert(sizeof(SegmentList) < 4000 && sizeof(PairList) < 4000 && sizeof(DiagList) < 4000,
+              "lists share the 4 KB of kernel parameters");
+
+// status of a host list of n entries
+int list_status(const void* h, int64_t n) {
+    if (n < 0 || (n > 0 && h == nullptr)) return FS_ERR_INVALID_ARG;
+    return n > FS_LIST_MAX ? FS_ERR_TOO_LARGE : FS_OK;
+}
+
 }  // namespace
 
 extern "C" int fs_weighted_sumsq(const double* d_x, const FsSegment* d_segs, int64_t n_segs,
                                  double* d_partial, int64_t n_partial, double* d_out,
                                  void* stream) {
-    return weighted_reduce<0>(d_x, d_segs, n_segs, d_partial, n_partial, d_out, stream);
+    if (n_segs < 0 || (n_segs > 0 && d_segs == nullptr)) return FS_ERR_INVALID_ARG;
+    return weighted_reduce<0>(d_x, fsb::DeviceTable<FsSegment>{d_segs}, n_segs, d_partial,
+                              n_partial, d_out, stream);
 }
 
 extern "C" int fs_weighted_sum(const double* d_x, const FsSegment* d_segs, int64_t n_segs,
                                double* d_partial, int64_t n_partial, double* d_out,
                                void* stream) {
-    return weighted_reduce<1>(d_x, d_segs, n_segs, d_partial, n_partial, d_out, stream);
+    if (n_segs < 0 || (n_segs > 0 && d_segs == nullptr)) return FS_ERR_INVALID_ARG;
+    return weighted_reduce<1>(d_x, fsb::DeviceTable<FsSegment>{d_segs}, n_segs, d_partial,
+                              n_partial, d_out, stream);
+}
+
+extern "C" int fs_weighted_sum_list(const double* d_x, const FsSegment* h_segs, int64_t n_segs,
+                                    int32_t squares, double* d_partial, int64_t n_partial,
+                                    double* d_out, void* stream) {
+    const int st = list_status(h_segs, n_segs);
+    if (st != FS_OK) return st;
+    const SegmentList t = fsb::inline_table<FsSegment, FS_LIST_MAX>(h_segs, n_segs);
+    return squares ? weighted_reduce<0>(d_x, t, n_segs, d_partial, n_partial, d_out, stream)
+                   : weighted_reduce<1>(d_x, t, n_segs, d_partial, n_partial, d_out, stream);
 }
 
 extern "C" int fs_pair_contract(const double* d_a, const double* d_b,
                                 const FsPairBlock* d_pairs, int64_t n_pairs,
                                 double* d_partial, int64_t n_partial, double* d_out,
                                 void* stream) {
-    if (n_pairs < 0 || n_partial < fsb::kReducePartials) return FS_ERR_INVALID_ARG;
-    if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
-    if (n_pairs > 0 && (d_a == nullptr || d_pairs == nullptr)) return FS_ERR_INVALID_ARG;
-    cudaStream_t s = fsb::as_stream(stream);
-    fsb::k_pair_contract<<<fsb::kReducePartials, fsb::kOpThreads, 0, s>>>(d_a, d_b, d_pairs,
-                                                                          n_pairs, d_partial);
-    int st = fsb::launch_status();
+    if (n_pairs < 0 || (n_pairs > 0 && d_pairs == nullptr)) return FS_ERR_INVALID_ARG;
+    return pair_contract(d_a, d_b, fsb::DeviceTable<FsPairBlock>{d_pairs}, n_pairs, d_partial,
+                         n_partial, d_out, stream);
+}
+
+extern "C" int fs_pair_contract_list(const double* d_a, const double* d_b,
+                                     const FsPairBlock* h_pairs, int64_t n_pairs,
+                                     double* d_partial, int64_t n_partial, double* d_out,
+                                     void* stream) {
+    const int st = list_status(h_pairs, n_pairs);
     if (st != FS_OK) return st;
-    fsb::k_final_sum<<<1, fsb::kOpThreads, 0, s>>>(d_partial, fsb::kReducePartials, d_out);
-    return fsb::launch_status();
+    return pair_contract(d_a, d_b, fsb::inline_table<FsPairBlock, FS_LIST_MAX>(h_pairs, n_pairs),
+                         n_pairs, d_partial, n_partial, d_out, stream);
 }
 
 extern "C" int fs_diag_mul(const double* d_x, const double* d_diag, double* d_out,
                            const FsDiagBlock* d_blocks, int64_t n_blocks, void* stream) {
     if (n_blocks < 0) return FS_ERR_INVALID_ARG;
     if (n_blocks == 0) return FS_OK;
-    if (d_x == nullptr || d_diag == nullptr || d_out == nullptr || d_blocks == nullptr)
-        return FS_ERR_INVALID_ARG;
-    // one wave of resident CTAs; CTAs without a unit return at once
-    fsb::k_diag_mul<<<4 * fsb::num_sms(), fsb::kOpThreads, 0, fsb::as_stream(stream)>>>(
-        d_x, d_diag, d_out, d_blocks, n_blocks);
-    return fsb::launch_status();
+    if (d_blocks == nullptr) return FS_ERR_INVALID_ARG;
+    return diag_mul(d_x, d_diag, d_out, fsb::DeviceTable<FsDiagBlock>{d_blocks}, n_blocks, stream);
+}
+
+extern "C" int fs_diag_mul_list(const double* d_x, const double* d_diag, double* d_out,
+                                const FsDiagBlock* h_blocks, int64_t n_blocks, void* stream) {
+    const int st = list_status(h_blocks, n_blocks);
+    if (st != FS_OK || n_blocks == 0) return st;
+    return diag_mul(d_x, d_diag, d_out,
+                    fsb::inline_table<FsDiagBlock, FS_LIST_MAX>(h_blocks, n_blocks), n_blocks,
+                    stream);
 }

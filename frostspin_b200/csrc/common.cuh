@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "../../include/frostspin_b200.h"
 
@@ -34,6 +35,30 @@ inline int launch_status() {
 }
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
+
+// A table of a launch: in device memory, or passed by value with the kernel's
+// parameters (the *_list entry points), which spares small launches the copies
+// to the device.  A product of 9 small sectors: 214 us of host time with its two
+// tables and the launch that expanded the tile list, 82 us with its problems in
+// the parameters.
+template <class T>
+struct DeviceTable {
+    const T* p;
+    __device__ __forceinline__ const T& operator[](int64_t i) const { return p[i]; }
+};
+
+template <class T, int N>
+struct InlineTable {
+    T v[N];
+    __device__ __forceinline__ const T& operator[](int64_t i) const { return v[i]; }
+};
+
+template <class T, int N>
+inline InlineTable<T, N> inline_table(const T* h, int64_t n) {
+    InlineTable<T, N> t;
+    memcpy(t.v, h, sizeof(T) * static_cast<size_t>(n));
+    return t;
+}
 
 // Granlund-Montgomery division by an invariant 32-bit divisor d:
 // q = (umulhi(n, m) + n) >> s with s = ceil(log2 d), m = floor(2^32 (2^s - d) / d) + 1.

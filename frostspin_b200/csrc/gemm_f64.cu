@@ -179,17 +179,75 @@ __device__ __forceinline__ void dgemm_tile(const FsGemmProblem& p, int m0, int n
     }
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 3)
-    k_grouped_dgemm(const FsGemmProblem* __restrict__ problems, int64_t n_problems,
-                    const FsGemmTile* __restrict__ tiles, int64_t n_tiles) {
-    extern __shared__ __align__(16) double smem[];
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+// Where a launch finds its problems and output tiles (TM x TN): a device table of
+// both, or problems passed with the kernel's parameters, whose tiles are
+// enumerated here -- problem by problem, column-major when a problem has more
+// tile columns than rows (its few row tiles then share each B column block in
+// L2).  `find` takes non-decreasing t for one cursor; false: an invalid entry.
+struct TileTable {
+    const FsGemmProblem* problems;
+    int64_t n_problems;
+    const FsGemmTile* tiles;
+    int64_t n_tiles;
+
+    struct Cursor {};
+    template <int TM, int TN>
+    __device__ __forceinline__ bool find(Cursor&, int64_t t, FsGemmProblem& p, int& m0,
+                                         int& n0) const {
         const FsGemmTile tile = tiles[t];
-        if (tile.problem < 0 || tile.problem >= n_problems) continue;
-        const FsGemmProblem p = problems[tile.problem];
-        const int m0 = tile.tm * kTM;
-        const int n0 = tile.tn * kTN;
-        if (m0 >= p.M || n0 >= p.N) continue;
+        if (tile.problem < 0 || tile.problem >= n_problems) return false;
+        p = problems[tile.problem];
+        m0 = tile.tm * TM;
+        n0 = tile.tn * TN;
+        return m0 < p.M && n0 < p.N;
+    }
+};
+
+template <int N>
+struct TileList {
+    FsGemmProblem v[N];
+    int64_t n_problems;
+    int64_t n_tiles;
+
+    struct Cursor {
+        int problem = 0;
+        int64_t first = 0;   // the problem's first tile
+    };
+    template <int TM, int TN>
+    __host__ __device__ __forceinline__ static int64_t count(const FsGemmProblem& p) {
+        return static_cast<int64_t>((p.M + TM - 1) / TM) * ((p.N + TN - 1) / TN);
+    }
+    template <int TM, int TN>
+    __device__ __forceinline__ bool find(Cursor& c, int64_t t, FsGemmProblem& p, int& m0,
+                                         int& n0) const {
+        int64_t n = count<TM, TN>(v[c.problem]);
+        while (t >= c.first + n) {
+            c.first += n;
+            n = count<TM, TN>(v[++c.problem]);
+        }
+        p = v[c.problem];
+        // keep the fields in registers: the compiler would read them from the
+        // parameters again for every k slice
+        asm volatile("" : "+l"(p.A), "+l"(p.B), "+l"(p.lda), "+l"(p.ldb), "+r"(p.M), "+r"(p.N), "+r"(p.K));
+        // a problem has fewer than 2^31 tiles (host)
+        const uint32_t k = static_cast<uint32_t>(t - c.first);
+        const uint32_t nr = (p.M + TM - 1) / TM, nc = (p.N + TN - 1) / TN;
+        const uint32_t q = k / (nc > nr ? nr : nc), r = k - q * (nc > nr ? nr : nc);
+        m0 = static_cast<int>(nc > nr ? r : q) * TM;
+        n0 = static_cast<int>(nc > nr ? q : r) * TN;
+        return true;
+    }
+};
+
+template <class Tiles>
+__global__ void __launch_bounds__(kGemmThreads, 3)
+    k_grouped_dgemm(const __grid_constant__ Tiles tiles) {
+    extern __shared__ __align__(16) double smem[];
+    typename Tiles::Cursor cursor;
+    for (int64_t t = blockIdx.x; t < tiles.n_tiles; t += gridDim.x) {
+        FsGemmProblem p;
+        int m0, n0;
+        if (!tiles.template find<kTM, kTN>(cursor, t, p, m0, n0)) continue;
         switch ((p.transA ? 2 : 0) | (p.transB ? 1 : 0)) {
             case 0: dgemm_tile<false, false>(p, m0, n0, smem); break;
             case 1: dgemm_tile<false, true>(p, m0, n0, smem); break;
@@ -207,37 +265,31 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
 // wholly outside the problem (M, N, K padding of the 64x64x16 tiling) issue no
 // DMMA.  Tiles of problems with K = 0 consume no stage (their output is
 // beta * C).
+template <class Tiles>
 struct TileCursor {
+    typename Tiles::Cursor at;
     int64_t t;
     FsGemmProblem p;
     int m0, n0, nk;
 };
 
-__device__ __forceinline__ bool cursor_seek(TileCursor& c, int64_t t,
-                                            const FsGemmProblem* __restrict__ problems,
-                                            int64_t n_problems,
-                                            const FsGemmTile* __restrict__ tiles, int64_t n_tiles,
+template <class Tiles>
+__device__ __forceinline__ bool cursor_seek(TileCursor<Tiles>& c, int64_t t, const Tiles& tiles,
                                             bool need_k) {
-    for (; t < n_tiles; t += gridDim.x) {
-        const FsGemmTile tile = tiles[t];
-        if (tile.problem < 0 || tile.problem >= n_problems) continue;
-        c.p = problems[tile.problem];
-        c.m0 = tile.tm * kTM;
-        c.n0 = tile.tn * kTN;
-        if (c.m0 >= c.p.M || c.n0 >= c.p.N) continue;
+    for (; t < tiles.n_tiles; t += gridDim.x) {
+        if (!tiles.template find<kTM, kTN>(c.at, t, c.p, c.m0, c.n0)) continue;
         c.nk = (c.p.K + kTK - 1) / kTK;
         if (need_k && c.nk == 0) continue;
         c.t = t;
         return true;
     }
-    c.t = n_tiles;
+    c.t = tiles.n_tiles;
     return false;
 }
 
-template <bool TA, bool TB>
+template <bool TA, bool TB, class Tiles>
 __global__ void __launch_bounds__(kGemmThreads, 3)
-    k_grouped_dgemm_stream(const FsGemmProblem* __restrict__ problems, int64_t n_problems,
-                           const FsGemmTile* __restrict__ tiles, int64_t n_tiles) {
+    k_grouped_dgemm_stream(const __grid_constant__ Tiles tiles) {
     extern __shared__ __align__(16) double smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -249,8 +301,8 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     const int b_off = TB ? (wn + fr) * kLdK + fk : fk * kLdR + wn + fr;
 
     // loader: the next (tile, k slice) to fetch; tiles without k slices skipped
-    TileCursor ld;
-    bool ld_ok = cursor_seek(ld, blockIdx.x, problems, n_problems, tiles, n_tiles, true);
+    TileCursor<Tiles> ld;
+    bool ld_ok = cursor_seek(ld, blockIdx.x, tiles, true);
     int ld_k = 0;
     int64_t issued = 0;
     auto issue = [&]() {
@@ -260,16 +312,15 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
             ++issued;
             if (++ld_k == ld.nk) {
                 ld_k = 0;
-                ld_ok = cursor_seek(ld, ld.t + gridDim.x, problems, n_problems, tiles, n_tiles,
-                                    true);
+                ld_ok = cursor_seek(ld, ld.t + gridDim.x, tiles, true);
             }
         }
         cp_async_commit();
     };
 
     // consumer: every tile of this CTA in order (K = 0 tiles included)
-    TileCursor cs;
-    bool cs_ok = cursor_seek(cs, blockIdx.x, problems, n_problems, tiles, n_tiles, false);
+    TileCursor<Tiles> cs;
+    bool cs_ok = cursor_seek(cs, blockIdx.x, tiles, false);
     int cs_k = 0;
     int64_t consumed = 0;
     double acc[4][4][2];
@@ -316,7 +367,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
             }
         }
         cs_k = 0;
-        cs_ok = cursor_seek(cs, cs.t + gridDim.x, problems, n_problems, tiles, n_tiles, false);
+        cs_ok = cursor_seek(cs, cs.t + gridDim.x, tiles, false);
     }
     cp_async_wait<0>();
 }
@@ -330,38 +381,50 @@ extern "C" int fs_dgemm_tile_shape(int32_t* tile_m, int32_t* tile_n) {
     return FS_OK;
 }
 
+namespace {
+
+inline int persistent_grid(int64_t n_tiles, int ctas) {
+    const int64_t max_grid = static_cast<int64_t>(fsb::num_sms()) * ctas;
+    return static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
+}
+
+template <class Tiles>
+int launch_tiles(const Tiles& tiles, cudaStream_t s) {
+    const int cfg = fsb::configure_smem(reinterpret_cast<const void*>(fsb::k_grouped_dgemm<Tiles>),
+                                        static_cast<int>(fsb::kGemmSmem));
+    if (cfg != FS_OK) return cfg;
+    fsb::k_grouped_dgemm<<<persistent_grid(tiles.n_tiles, 3), fsb::kGemmThreads, fsb::kGemmSmem,
+                           s>>>(tiles);
+    return fsb::launch_status();
+}
+
+template <bool TA, bool TB, class Tiles>
+int launch_stream_t(const Tiles& tiles, cudaStream_t s) {
+    const int cfg = fsb::configure_smem(
+        reinterpret_cast<const void*>(fsb::k_grouped_dgemm_stream<TA, TB, Tiles>),
+        static_cast<int>(fsb::kGemmSmem));
+    if (cfg != FS_OK) return cfg;
+    fsb::k_grouped_dgemm_stream<TA, TB><<<persistent_grid(tiles.n_tiles, 3), fsb::kGemmThreads,
+                                          fsb::kGemmSmem, s>>>(tiles);
+    return fsb::launch_status();
+}
+
+template <class Tiles>
+int launch_stream(const Tiles& tiles, bool ta, bool tb, cudaStream_t s) {
+    if (ta) return tb ? launch_stream_t<true, true>(tiles, s) : launch_stream_t<true, false>(tiles, s);
+    return tb ? launch_stream_t<false, true>(tiles, s) : launch_stream_t<false, false>(tiles, s);
+}
+
+}  // namespace
+
 extern "C" int fs_grouped_dgemm(const FsGemmProblem* d_problems, int64_t n_problems,
                                 const FsGemmTile* d_tiles, int64_t n_tiles, void* stream) {
     if (n_tiles < 0 || n_problems < 0) return FS_ERR_INVALID_ARG;
     if (n_tiles == 0) return FS_OK;
     if (d_problems == nullptr || d_tiles == nullptr) return FS_ERR_INVALID_ARG;
-    const int cfg = fsb::configure_smem(reinterpret_cast<const void*>(fsb::k_grouped_dgemm),
-                                        static_cast<int>(fsb::kGemmSmem));
-    if (cfg != FS_OK) return cfg;
-    const int64_t max_grid = static_cast<int64_t>(fsb::num_sms()) * 3;
-    const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    fsb::k_grouped_dgemm<<<grid, fsb::kGemmThreads, fsb::kGemmSmem, fsb::as_stream(stream)>>>(
-        d_problems, n_problems, d_tiles, n_tiles);
-    return fsb::launch_status();
+    return launch_tiles(fsb::TileTable{d_problems, n_problems, d_tiles, n_tiles},
+                        fsb::as_stream(stream));
 }
-
-namespace {
-
-template <bool TA, bool TB>
-int launch_stream(const FsGemmProblem* d_problems, int64_t n_problems, const FsGemmTile* d_tiles,
-                  int64_t n_tiles, cudaStream_t s) {
-    const int cfg = fsb::configure_smem(
-        reinterpret_cast<const void*>(fsb::k_grouped_dgemm_stream<TA, TB>),
-        static_cast<int>(fsb::kGemmSmem));
-    if (cfg != FS_OK) return cfg;
-    const int64_t max_grid = static_cast<int64_t>(fsb::num_sms()) * 3;
-    const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    fsb::k_grouped_dgemm_stream<TA, TB><<<grid, fsb::kGemmThreads, fsb::kGemmSmem, s>>>(
-        d_problems, n_problems, d_tiles, n_tiles);
-    return fsb::launch_status();
-}
-
-}  // namespace
 
 extern "C" int fs_grouped_dgemm_uniform(const FsGemmProblem* d_problems, int64_t n_problems,
                                         const FsGemmTile* d_tiles, int64_t n_tiles,
@@ -369,12 +432,8 @@ extern "C" int fs_grouped_dgemm_uniform(const FsGemmProblem* d_problems, int64_t
     if (n_tiles < 0 || n_problems < 0) return FS_ERR_INVALID_ARG;
     if (n_tiles == 0) return FS_OK;
     if (d_problems == nullptr || d_tiles == nullptr) return FS_ERR_INVALID_ARG;
-    cudaStream_t s = fsb::as_stream(stream);
-    if (trans_a)
-        return trans_b ? launch_stream<true, true>(d_problems, n_problems, d_tiles, n_tiles, s)
-                       : launch_stream<true, false>(d_problems, n_problems, d_tiles, n_tiles, s);
-    return trans_b ? launch_stream<false, true>(d_problems, n_problems, d_tiles, n_tiles, s)
-                   : launch_stream<false, false>(d_problems, n_problems, d_tiles, n_tiles, s);
+    return launch_stream(fsb::TileTable{d_problems, n_problems, d_tiles, n_tiles}, trans_a != 0,
+                         trans_b != 0, fsb::as_stream(stream));
 }
 
 // ---------------------------------------------------------------- thin GEMMs
@@ -451,19 +510,21 @@ __device__ __forceinline__ void thin_tile_k(const FsGemmProblem& p, const double
         thin_tile<MB, 32, 1>(p, su, n0);
 }
 
+template <class Tiles>
 __global__ void __launch_bounds__(kThinThreads, 4)
-    k_grouped_dgemm_thin(const FsGemmProblem* __restrict__ problems, int64_t n_problems,
-                         const FsGemmTile* __restrict__ tiles, int64_t n_tiles) {
+    k_grouped_dgemm_thin(const __grid_constant__ Tiles tiles) {
     __shared__ double su[kThinMax * kThinMax];
     constexpr int kCols = kThinThreads * kThinColsPerThread;
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        const FsGemmTile tile = tiles[t];
-        if (tile.problem < 0 || tile.problem >= n_problems) continue;
-        const FsGemmProblem p = problems[tile.problem];
-        if (p.M > kThinMax || p.K > kThinMax || p.transA || p.transB) continue;
-        const int n0 = tile.tn * kCols;
-        if (n0 >= p.N) continue;
-        __syncthreads();  // previous tile's reads of su are done
+    __shared__ FsGemmProblem p;   // in registers beside the operands it spills
+    typename Tiles::Cursor cursor;
+    for (int64_t t = blockIdx.x; t < tiles.n_tiles; t += gridDim.x) {
+        FsGemmProblem found;
+        int m0, n0;   // every row is in one tile; tables leave tm at 0
+        if (!tiles.template find<kThinMax, kCols>(cursor, t, found, m0, n0)) continue;
+        if (found.M > kThinMax || found.K > kThinMax || found.transA || found.transB) continue;
+        __syncthreads();  // previous tile's reads of su and p are done
+        if (threadIdx.x == 0) p = found;
+        __syncthreads();
         // rows m < M of U, zero-padded to kThinMax columns (the unrolled k
         // loop reads up to K rounded up)
         const int mk = p.M * kThinMax;
@@ -493,16 +554,72 @@ extern "C" int fs_thin_dgemm_shape(int32_t* max_m, int32_t* max_k, int32_t* tile
     return FS_OK;
 }
 
+namespace {
+
+template <class Tiles>
+int launch_thin(const Tiles& tiles, cudaStream_t s) {
+    fsb::k_grouped_dgemm_thin<<<persistent_grid(tiles.n_tiles, 8), fsb::kThinThreads, 0, s>>>(
+        tiles);
+    return fsb::launch_status();
+}
+
+}  // namespace
+
 extern "C" int fs_grouped_dgemm_thin(const FsGemmProblem* d_problems, int64_t n_problems,
                                      const FsGemmTile* d_tiles, int64_t n_tiles, void* stream) {
     if (n_tiles < 0 || n_problems < 0) return FS_ERR_INVALID_ARG;
     if (n_tiles == 0) return FS_OK;
     if (d_problems == nullptr || d_tiles == nullptr) return FS_ERR_INVALID_ARG;
-    const int64_t max_grid = static_cast<int64_t>(fsb::num_sms()) * 8;
-    const int grid = static_cast<int>(n_tiles < max_grid ? n_tiles : max_grid);
-    fsb::k_grouped_dgemm_thin<<<grid, fsb::kThinThreads, 0, fsb::as_stream(stream)>>>(
-        d_problems, n_problems, d_tiles, n_tiles);
-    return fsb::launch_status();
+    return launch_thin(fsb::TileTable{d_problems, n_problems, d_tiles, n_tiles},
+                       fsb::as_stream(stream));
+}
+
+namespace {
+
+// Problems by value: 3.5 KB of parameters, or 31 KB for longer lists.
+template <int N>
+int launch_list(const FsGemmProblem* h, int64_t n, int kind, cudaStream_t s) {
+    fsb::TileList<N> t;
+    memcpy(t.v, h, sizeof(FsGemmProblem) * static_cast<size_t>(n));
+    t.n_problems = n;
+    t.n_tiles = 0;
+    constexpr int kThinCols = fsb::kThinThreads * fsb::kThinColsPerThread;
+    for (int64_t i = 0; i < n; ++i) {
+        const FsGemmProblem& p = h[i];
+        if (p.M < 0 || p.N < 0 || p.K < 0) return FS_ERR_INVALID_ARG;
+        const int64_t tiles =
+            kind == FS_DGEMM_THIN
+                ? fsb::TileList<N>::template count<fsb::kThinMax, kThinCols>(p)
+                : fsb::TileList<N>::template count<fsb::kTM, fsb::kTN>(p);
+        if (tiles >= (1ll << 31)) return FS_ERR_TOO_LARGE;
+        t.n_tiles += tiles;
+        if (kind == FS_DGEMM_UNIFORM && ((p.transA != 0) != (h[0].transA != 0) ||
+                                         (p.transB != 0) != (h[0].transB != 0)))
+            return FS_ERR_INVALID_ARG;
+        if (kind == FS_DGEMM_THIN &&
+            (p.M > fsb::kThinMax || p.K > fsb::kThinMax || p.transA || p.transB))
+            return FS_ERR_INVALID_ARG;
+    }
+    if (t.n_tiles == 0) return FS_OK;
+    if (kind == FS_DGEMM_TILES) return launch_tiles(t, s);
+    if (kind == FS_DGEMM_UNIFORM) return launch_stream(t, h[0].transA != 0, h[0].transB != 0, s);
+    return launch_thin(t, s);
+}
+
+}  // namespace
+
+extern "C" int fs_grouped_dgemm_list(const FsGemmProblem* h_problems, int64_t n_problems,
+                                     int32_t kind, void* stream) {
+    constexpr int kShort = 40;
+    static_assert(sizeof(fsb::TileList<kShort>) < 4000, "short lists fit 4 KB of parameters");
+    static_assert(sizeof(fsb::TileList<FS_DGEMM_LIST_MAX>) <= 32764, "kernel parameter limit");
+    if (n_problems < 0 || kind < FS_DGEMM_TILES || kind > FS_DGEMM_THIN) return FS_ERR_INVALID_ARG;
+    if (n_problems == 0) return FS_OK;
+    if (h_problems == nullptr) return FS_ERR_INVALID_ARG;
+    if (n_problems > FS_DGEMM_LIST_MAX) return FS_ERR_TOO_LARGE;
+    cudaStream_t s = fsb::as_stream(stream);
+    return n_problems <= kShort ? launch_list<kShort>(h_problems, n_problems, kind, s)
+                                : launch_list<FS_DGEMM_LIST_MAX>(h_problems, n_problems, kind, s);
 }
 
 // ------------------------------------------------------------ split-K reduce
@@ -512,8 +629,9 @@ extern "C" int fs_grouped_dgemm_thin(const FsGemmProblem* d_problems, int64_t n_
 // in order (deterministic, no atomics) and applies alpha / beta into C.
 namespace fsb {
 
+template <class Table>
 __global__ void __launch_bounds__(256)
-    k_splitk_reduce(const FsSplitReduce* __restrict__ items, int64_t n_items) {
+    k_splitk_reduce(const __grid_constant__ Table items, int64_t n_items) {
     const int64_t it = blockIdx.y;
     if (it >= n_items) return;
     const FsSplitReduce r = items[it];
@@ -530,17 +648,36 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace fsb
 
+namespace {
+
+template <class Table>
+int splitk_reduce(const Table& items, int64_t n_items, int64_t max_elems, void* stream) {
+    const int64_t blocks = (max_elems + 255) / 256;
+    const int gx = static_cast<int>(blocks < 4 * fsb::num_sms() ? blocks : 4 * fsb::num_sms());
+    fsb::k_splitk_reduce<<<dim3(gx, static_cast<unsigned>(n_items)), 256, 0,
+                           fsb::as_stream(stream)>>>(items, n_items);
+    return fsb::launch_status();
+}
+
+}  // namespace
+
 extern "C" int fs_splitk_reduce(const FsSplitReduce* d_items, int64_t n_items,
                                 int64_t max_elems, void* stream) {
     if (n_items < 0 || max_elems < 0) return FS_ERR_INVALID_ARG;
     if (n_items == 0 || max_elems == 0) return FS_OK;
     if (d_items == nullptr) return FS_ERR_INVALID_ARG;
     if (n_items > 65535) return FS_ERR_TOO_LARGE;
-    const int64_t blocks = (max_elems + 255) / 256;
-    const int gx = static_cast<int>(blocks < 4 * fsb::num_sms() ? blocks : 4 * fsb::num_sms());
-    fsb::k_splitk_reduce<<<dim3(gx, static_cast<unsigned>(n_items)), 256, 0,
-                           fsb::as_stream(stream)>>>(d_items, n_items);
-    return fsb::launch_status();
+    return splitk_reduce(fsb::DeviceTable<FsSplitReduce>{d_items}, n_items, max_elems, stream);
+}
+
+extern "C" int fs_splitk_reduce_list(const FsSplitReduce* h_items, int64_t n_items,
+                                     int64_t max_elems, void* stream) {
+    if (n_items < 0 || max_elems < 0) return FS_ERR_INVALID_ARG;
+    if (n_items == 0 || max_elems == 0) return FS_OK;
+    if (h_items == nullptr) return FS_ERR_INVALID_ARG;
+    if (n_items > FS_SPLIT_LIST_MAX) return FS_ERR_TOO_LARGE;
+    return splitk_reduce(fsb::inline_table<FsSplitReduce, FS_SPLIT_LIST_MAX>(h_items, n_items),
+                         n_items, max_elems, stream);
 }
 
 // Tile table from runs (see FsTileRun): one thread per tile, binary search of

@@ -21,6 +21,7 @@ from . import _native  # noqa: E402
 
 _scratch = {}
 _available = []
+_devices = {}
 
 
 def device():
@@ -31,12 +32,16 @@ def device():
             msg = "frostspin_b200 needs a CUDA device (B200, sm_100a); none is available"
             raise RuntimeError(msg)
         _available.append(True)
-    return torch.device("cuda", torch.cuda.current_device())
+    index = torch.cuda.current_device()
+    d = _devices.get(index)
+    if d is None:
+        d = _devices[index] = torch.device("cuda", index)
+    return d
 
 
 def stream():
     """cudaStream_t of torch's current stream, as an integer handle."""
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t):

@@ -23,11 +23,19 @@ def disable():
     _state["on"] = False
 
 
-@contextlib.contextmanager
+_OFF = contextlib.nullcontext()
+
+
+def enabled():
+    return _state["on"]
+
+
 def region(name, **work):
-    if not _state["on"]:
-        yield
-        return
+    return _timed(name, work) if _state["on"] else _OFF
+
+
+@contextlib.contextmanager
+def _timed(name, work):
     s = torch.cuda.Event(enable_timing=True)
     e = torch.cuda.Event(enable_timing=True)
     s.record()

@@ -114,7 +114,7 @@ def shared_launches():
         if pend["perm"]:
             _flush_permutes(pend["perm"])
         if pend["gemm"]:
-            grouped_gemm(pend["gemm"])
+            run_gemm_table(np.concatenate([arr for arr, _ in pend["gemm"]]), pend["gemm"])
     finally:
         _SHARED = old
 
@@ -214,38 +214,59 @@ def grouped_gemm(problems):
     are C-order (ldc = N).  A with a_trans False is C-order M x K (lda = K);
     with a_trans True it is stored K x M (lda = M).  Likewise for B.
     """
-    n = len(problems)
-    if n == 0:
+    arr = np.zeros(len(problems), dtype=_native.GEMM_PROBLEM_DTYPE)
+    rows = []
+    for p in problems:
+        M, N, K = int(p["M"]), int(p["N"]), int(p["K"])
+        rows.append((
+            p["A"].data_ptr() + 8 * int(p["a_off"]), p["B"].data_ptr() + 8 * int(p["b_off"]),
+            p["C"].data_ptr() + 8 * int(p["c_off"]),
+            p.get("lda", M if p["a_trans"] else K), p.get("ldb", K if p["b_trans"] else N), N,
+            M, N, K, bool(p["a_trans"]), bool(p["b_trans"]), 0, p.get("alpha", 1.0),
+            p.get("beta", 0.0),
+        ))
+    if rows:
+        arr[:] = rows
+    run_gemm_table(arr, problems)
+
+
+def block_gemm(a, a_off, a_trans, b, b_off, b_trans, c, c_off, M, N, K):
+    """C_i = op(A_i) op(B_i) for blocks of three buffers: element offsets and
+    sizes as int64 arrays, C-order results, one launch (see grouped_gemm)."""
+    arr = np.zeros(len(M), dtype=_native.GEMM_PROBLEM_DTYPE)
+    arr["A"] = a.data_ptr() + 8 * a_off
+    arr["B"] = b.data_ptr() + 8 * b_off
+    arr["C"] = c.data_ptr() + 8 * c_off
+    arr["lda"] = M if a_trans else K
+    arr["ldb"] = K if b_trans else N
+    arr["ldc"] = N
+    arr["M"], arr["N"], arr["K"] = M, N, K
+    arr["transA"], arr["transB"] = a_trans, b_trans
+    arr["alpha"] = 1.0
+    run_gemm_table(arr, (a, b, c))
+
+
+def _flops(arr):
+    return float((2.0 * arr["M"].astype(np.float64) * arr["N"] * arr["K"]).sum())
+
+
+def run_gemm_table(arr, keep=None):
+    """Run an FsGemmProblem table at the current GEMM precision; inside
+    shared_launches it is queued, with the buffers `keep` it points into."""
+    if arr.size == 0:
         return
     if _SHARED is not None:
-        _SHARED["gemm"].extend(problems)
+        _SHARED["gemm"].append((arr, keep))
         return
-    arr = np.zeros(n, dtype=_native.GEMM_PROBLEM_DTYPE)
-    tm, tn = _tile_shape()
-    ntile = []
-    for i, p in enumerate(problems):
-        M, N, K = int(p["M"]), int(p["N"]), int(p["K"])
-        arr["A"][i] = p["A"].data_ptr() + 8 * int(p["a_off"])
-        arr["B"][i] = p["B"].data_ptr() + 8 * int(p["b_off"])
-        arr["C"][i] = p["C"].data_ptr() + 8 * int(p["c_off"])
-        arr["lda"][i] = p.get("lda", M if p["a_trans"] else K)
-        arr["ldb"][i] = p.get("ldb", K if p["b_trans"] else N)
-        arr["ldc"][i] = N
-        arr["M"][i], arr["N"][i], arr["K"][i] = M, N, K
-        arr["transA"][i] = int(bool(p["a_trans"]))
-        arr["transB"][i] = int(bool(p["b_trans"]))
-        arr["alpha"][i] = p.get("alpha", 1.0)
-        arr["beta"][i] = p.get("beta", 0.0)
-        ntile.append(((M + tm - 1) // tm) * ((N + tn - 1) // tn))
     if _RECORDER is not None:
         _RECORDER.append(arr.copy())
     mode = gemm_precision()
-    ntile = np.array(ntile, dtype=np.int64)
-    flops = 2.0 * (arr["M"].astype(np.float64) * arr["N"] * arr["K"])
+    timed = instrument.enabled()
     if mode == "fp64":
-        with instrument.region("gemm_fp64", flops=float(flops.sum())):
-            _dgemm(arr, problems, tm, tn, ntile)
-    elif mode.startswith("ozaki2_"):
+        with instrument.region("gemm_fp64", flops=_flops(arr) if timed else 0.0):
+            _dgemm(arr)
+        return
+    if mode.startswith("ozaki2_"):
         nmod = int(mode[7:])
         fits = arr["K"].astype(np.int64) <= _native.FS_OZAKI2_MAX_K
         if _PRECISION["dispatch"] == "all":
@@ -254,11 +275,8 @@ def grouped_gemm(problems):
             use = fits & _tuned(arr, mode, ozaki2_pays(arr, nmod))
         if use.any():
             # regions inside: the split kernels and the tcgen05 GEMM apart
-            ozaki2_gemm(arr[use], nmod, flops=float(flops[use].sum()),
+            ozaki2_gemm(arr[use], nmod, flops=_flops(arr[use]),
                         int8_ops=ozaki2_int8_ops(arr[use], nmod))
-        if (~use).any():
-            with instrument.region("gemm_fp64", flops=float(flops[~use].sum())):
-                _dgemm(arr[~use], None, tm, tn, ntile[~use])
     elif mode.startswith("ozaki"):
         S = int(mode[5:])
         if _PRECISION["dispatch"] == "all":
@@ -266,14 +284,14 @@ def grouped_gemm(problems):
         else:
             use = _tuned(arr, mode, ozaki_pays(arr, S))
         if use.any():
-            with instrument.region("gemm_ozaki", flops=float(flops[use].sum()),
+            with instrument.region("gemm_ozaki", flops=_flops(arr[use]),
                                    int8_ops=ozaki_int8_ops(arr[use], S)):
                 ozaki_gemm(arr[use], S)
-        if (~use).any():
-            with instrument.region("gemm_fp64", flops=float(flops[~use].sum())):
-                _dgemm(arr[~use], None, tm, tn, ntile[~use])
     else:  # pragma: no cover - guarded by set_gemm_precision
         raise ValueError(mode)
+    if not use.all():
+        with instrument.region("gemm_fp64", flops=_flops(arr[~use])):
+            _dgemm(arr[~use])
 
 
 _THIN = None
@@ -293,28 +311,27 @@ def grouped_dgemm_table(arr, region="gemm_fp64"):
     if arr.size == 0:
         return
     max_m, max_k, thin_n = _thin_shape()
-    M = arr["M"].astype(np.int64)
-    N = arr["N"].astype(np.int64)
-    K = arr["K"].astype(np.int64)
-    thin = (M <= max_m) & (K <= max_k) & (arr["transA"] == 0) & (arr["transB"] == 0)
-    if thin.any():
-        sub = arr[thin]
-        nt = (N[thin] + thin_n - 1) // thin_n
-        runs, total = _tile_runs(nt, nt, np.arange(sub.size))
-        d_prob = dev.upload(sub)
-        d_tiles = _device_tiles(runs, total)
-        flops = 2.0 * float((M[thin].astype(np.float64) * N[thin] * K[thin]).sum())
-        with instrument.region(region + "_thin", flops=flops,
-                               bytes=8.0 * float((N[thin] * (M[thin] + K[thin])).sum())):
-            _native.call("fs_grouped_dgemm_thin", d_prob.data_ptr(), sub.size,
-                         d_tiles.data_ptr(), total, dev.stream())
-    if (~thin).any():
-        sub = arr[~thin]
-        tm, tn = _tile_shape()
-        ntile = ((M[~thin] + tm - 1) // tm) * ((N[~thin] + tn - 1) // tn)
-        flops = 2.0 * float((M[~thin].astype(np.float64) * N[~thin] * K[~thin]).sum())
-        with instrument.region(region, flops=flops):
-            _dgemm(sub, None, tm, tn, ntile)
+    thin = ((arr["M"] <= max_m) & (arr["K"] <= max_k) & (arr["transA"] == 0)
+            & (arr["transB"] == 0))
+    n_thin = int(np.count_nonzero(thin))
+    if n_thin:
+        sub = arr if n_thin == arr.size else arr[thin]
+        M, N, K = (sub[k].astype(np.int64) for k in ("M", "N", "K"))
+        with instrument.region(region + "_thin", flops=2.0 * float((M * N * K).sum()),
+                               bytes=8.0 * float((N * (M + K)).sum())):
+            if sub.size <= _native.FS_DGEMM_LIST_MAX:
+                _dgemm_list("fs_grouped_dgemm_thin", sub, _native.FS_DGEMM_THIN)
+            else:
+                nt = (N + thin_n - 1) // thin_n
+                runs, total = _tile_runs(nt, nt, np.arange(sub.size))
+                d_prob = dev.upload(sub)
+                d_tiles = _device_tiles(runs, total)
+                _native.call("fs_grouped_dgemm_thin", d_prob.data_ptr(), sub.size,
+                             d_tiles.data_ptr(), total, dev.stream())
+    if n_thin < arr.size:
+        sub = arr[~thin] if n_thin else arr
+        with instrument.region(region, flops=_flops(sub) if instrument.enabled() else 0.0):
+            _dgemm(sub)
 
 
 # rates of the two paths on B200 inside the SU(2) CTMRG workload (int8: the
@@ -426,12 +443,15 @@ _SPLITK_CHUNK = 1024        # smallest K chunk of a split problem
 _SPLITK_TARGET_TILES = 3 * 148 * 2   # two waves of 3 CTAs per SM
 
 
-def _split_k(arr, tm, tn, ntile):
+def _split_k(arr):
     """Cut long-K problems of a launch that has too few output tiles into K
     chunks writing partial products to a workspace; returns the new problem
-    table and tile counts, the reduction items and the workspace (or None
-    when the launch already fills the GPU)."""
-    total = int(ntile.sum())
+    table, the reduction items and the workspace (or None when the launch
+    already fills the GPU)."""
+    if int(arr["K"].max(initial=0)) < 2 * _SPLITK_CHUNK:
+        return None
+    tm, tn = _tile_shape()
+    total = int(_tile_counts(arr, tm, tn).sum())
     if total == 0 or total >= _SPLITK_TARGET_TILES:
         return None
     factor = min(16, -(-_SPLITK_TARGET_TILES // total))
@@ -470,22 +490,56 @@ def _split_k(arr, tm, tn, ntile):
         items[n_items] = (base + 8 * int(w_off[i]), arr["C"][i], arr["ldc"][i], M[i] * N[i],
                           starts.size, M[i], N[i], 0, arr["alpha"][i], arr["beta"][i])
         n_items += 1
-    new = np.concatenate(rows)
-    nt = ((new["M"].astype(np.int64) + tm - 1) // tm) * ((new["N"].astype(np.int64) + tn - 1) // tn)
-    return new, nt, items[:n_items], work
+    return np.concatenate(rows), items[:n_items], work
+
+
+def _tile_counts(arr, tm, tn):
+    M = arr["M"].astype(np.int64)
+    N = arr["N"].astype(np.int64)
+    return ((M + tm - 1) // tm) * ((N + tn - 1) // tn)
 
 
 _STREAM_MAX_K = 256   # longest K of a launch that goes to the streaming kernel
 
 
-def _launch_dgemm(arr, d_prob, d_tiles, n_tiles):
+# The tables cost the host about 60 us and the device 8 us, hidden once a launch
+# runs longer than that; the per-tile kernel itself is 0.6 % faster with them
+# (10 335 tiles of K up to 2900: 6.81 ms with tables, 6.86 by value; 1008 tiles
+# 227 us both).  The streaming kernel is faster by value (wide sectors 313 us,
+# with tables 336 us).
+_LIST_TILES = 4 * 3 * 148
+
+
+def _dgemm_list(name, arr, kind):
+    """Launch kernel `name` with the problems passed by value, longest K first
+    (long tiles start early in the static schedule)."""
+    arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
+    _native.call(name, arr.ctypes.data, arr.size, kind, dev.stream(),
+                 entry="fs_grouped_dgemm_list")
+
+
+def _launch_dgemm(arr):
     """One DMMA launch over a problem table: the streaming kernel when every
     problem has the same transpose flags and a short K (pipeline fill and
     padded fragments dominate there), else the per-tile kernel (faster on long
-    K, where it keeps a few registers more for the DMMA loop)."""
+    K, where it keeps a few registers more for the DMMA loop).  Up to
+    FS_DGEMM_LIST_MAX problems travel with the launch; longer tables, and
+    launches of the per-tile kernel beyond _LIST_TILES tiles, go through device
+    memory with their tile list."""
     ta, tb = arr["transA"], arr["transB"]
-    if (arr.size and (ta == ta[0]).all() and (tb == tb[0]).all()
-            and int(arr["K"].max()) <= _STREAM_MAX_K):
+    uniform = ((ta == ta[0]).all() and (tb == tb[0]).all()
+               and int(arr["K"].max()) <= _STREAM_MAX_K)
+    tm, tn = _tile_shape()
+    counts = _tile_counts(arr, tm, tn)
+    if arr.size <= _native.FS_DGEMM_LIST_MAX and (uniform or int(counts.sum()) <= _LIST_TILES):
+        if uniform:
+            _dgemm_list("fs_grouped_dgemm_uniform", arr, _native.FS_DGEMM_UNIFORM)
+        else:
+            _dgemm_list("fs_grouped_dgemm", arr, _native.FS_DGEMM_TILES)
+        return
+    d_tiles, n_tiles = _tile_table(arr, tm, tn, counts)
+    d_prob = dev.upload(arr)
+    if uniform:
         _native.call("fs_grouped_dgemm_uniform", d_prob.data_ptr(), arr.size,
                      d_tiles.data_ptr(), n_tiles, int(ta[0]), int(tb[0]), dev.stream())
     else:
@@ -493,24 +547,23 @@ def _launch_dgemm(arr, d_prob, d_tiles, n_tiles):
                      n_tiles, dev.stream())
 
 
-def _dgemm(arr, problems, tm, tn, ntile):
-    sk = _split_k(arr, tm, tn, ntile)
-    if sk is not None:
-        arr, ntile, items, work = sk
-        d_tiles, n_tiles = _tile_table(arr, tm, tn, ntile)
-        d_prob = dev.upload(arr)
-        _launch_dgemm(arr, d_prob, d_tiles, n_tiles)
-        d_items = dev.upload(items)
-        max_elems = int((items["M"].astype(np.int64) * items["N"]).max())
-        for start in range(0, items.size, 65535):
-            cnt = min(65535, items.size - start)
-            _native.call("fs_splitk_reduce", d_items.data_ptr() + start * items.itemsize, cnt,
-                         max_elems, dev.stream())
-        return d_prob, d_tiles, work
-    d_tiles, n_tiles = _tile_table(arr, tm, tn, ntile)
-    d_prob = dev.upload(arr)
-    _launch_dgemm(arr, d_prob, d_tiles, n_tiles)
-    return d_prob, d_tiles
+def _dgemm(arr):
+    sk = _split_k(arr)
+    if sk is None:
+        _launch_dgemm(arr)
+        return
+    arr, items, _work = sk   # the workspace lives until the reduction is queued
+    _launch_dgemm(arr)
+    max_elems = int((items["M"].astype(np.int64) * items["N"]).max())
+    if items.size <= _native.FS_SPLIT_LIST_MAX:
+        _native.call("fs_splitk_reduce", items.ctypes.data, items.size, max_elems, dev.stream(),
+                     entry="fs_splitk_reduce_list")
+        return
+    d_items = dev.upload(items)
+    for start in range(0, items.size, 65535):
+        cnt = min(65535, items.size - start)
+        _native.call("fs_splitk_reduce", d_items.data_ptr() + start * items.itemsize, cnt,
+                     max_elems, dev.stream())
 
 
 def _operand(t):
@@ -539,26 +592,20 @@ def matmul_blocks(lefts, rights, *, alpha=1.0):
     if n > 1:
         offsets[1:] = np.cumsum(sizes[:-1])
     out = dev.empty_f64(int(sizes.sum()))
-    problems = []
-    keep = []
+    rows, keep = [], []
+    base = out.data_ptr()
     for i, (a, b) in enumerate(zip(lefts, rights, strict=True)):
         if a.shape[1] != b.shape[0]:
             raise ValueError("inner dimensions do not match")
         ta, lda, a_t = _operand(a)
         tb, ldb, b_t = _operand(b)
         keep += [ta, tb]
-        problems.append({
-            "A": ta, "a_off": 0, "a_trans": a_t, "lda": lda,
-            "B": tb, "b_off": 0, "b_trans": b_t, "ldb": ldb,
-            "C": out, "c_off": offsets[i], "M": a.shape[0], "N": b.shape[1],
-            "K": a.shape[1], "alpha": alpha,
-        })
-    for p in problems:
+        N = b.shape[1]
         # data_ptr() of a view already includes its storage offset
-        p["a_off"] = 0
-        p["b_off"] = 0
-    if problems:
-        grouped_gemm(problems)
+        rows.append((ta.data_ptr(), tb.data_ptr(), base + 8 * int(offsets[i]), lda, ldb, N,
+                     a.shape[0], N, a.shape[1], a_t, b_t, 0, alpha, 0.0))
+    if rows:
+        run_gemm_table(np.array(rows, dtype=_native.GEMM_PROBLEM_DTYPE), (out, keep))
     views = [out[o : o + m * k].view(m, k) for o, (m, k) in zip(offsets, shapes, strict=True)]
     return out, offsets, shapes, views
 
@@ -816,8 +863,13 @@ def weighted_reduce(buf, offsets, lengths, weights, *, squares):
     segs["length"] = lengths
     segs["weight"] = weights
     part = dev.scratch_partials()
-    d_segs = dev.upload(segs)
     name = "fs_weighted_sumsq" if squares else "fs_weighted_sum"
+    if segs.size <= _native.FS_LIST_MAX:
+        _native.call(name, dev.ptr(buf), segs.ctypes.data, segs.size, int(squares),
+                     part.data_ptr(), part.numel(), out.data_ptr(), dev.stream(),
+                     entry="fs_weighted_sum_list")
+        return out[0]
+    d_segs = dev.upload(segs)
     _native.call(
         name,
         dev.ptr(buf),
@@ -836,14 +888,20 @@ def pair_contract(abuf, bbuf, pairs):
     means trace of the A block.  Returns a 0-d device tensor."""
     out = torch.empty(1, dtype=torch.float64, device=abuf.device)
     tab = np.zeros(len(pairs), dtype=_native.PAIR_BLOCK_DTYPE)
-    for i, (ao, bo, m, n, at, bt, w) in enumerate(pairs):
-        tab[i] = (ao, bo, m, n, int(at), int(bt), w)
+    if len(pairs):
+        tab[:] = [tuple(p) for p in pairs]
     part = dev.scratch_partials()
+    b_ptr = dev.ptr(bbuf) if bbuf is not None else None
+    if tab.size <= _native.FS_LIST_MAX:
+        _native.call("fs_pair_contract", dev.ptr(abuf), b_ptr, tab.ctypes.data, tab.size,
+                     part.data_ptr(), part.numel(), out.data_ptr(), dev.stream(),
+                     entry="fs_pair_contract_list")
+        return out[0]
     d_tab = dev.upload(tab)
     _native.call(
         "fs_pair_contract",
         dev.ptr(abuf),
-        dev.ptr(bbuf) if bbuf is not None else None,
+        b_ptr,
         d_tab.data_ptr(),
         tab.size,
         part.data_ptr(),
@@ -887,8 +945,12 @@ def diag_mul(xbuf, dbuf, entries, out_len):
     """entries: list of (x_off, out_off, d_off, m, n, x_trans, left)."""
     out = dev.empty_f64(out_len)
     tab = np.zeros(len(entries), dtype=_native.DIAG_BLOCK_DTYPE)
-    for i, e in enumerate(entries):
-        tab[i] = (e[0], e[1], e[2], e[3], e[4], int(e[5]), int(e[6]))
+    if len(entries):
+        tab[:] = [tuple(e) for e in entries]
+    if tab.size <= _native.FS_LIST_MAX:
+        _native.call("fs_diag_mul", dev.ptr(xbuf), dev.ptr(dbuf), dev.ptr(out), tab.ctypes.data,
+                     tab.size, dev.stream(), entry="fs_diag_mul_list")
+        return out
     d_tab = dev.upload(tab)
     _native.call(
         "fs_diag_mul",

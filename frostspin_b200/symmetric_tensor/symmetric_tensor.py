@@ -442,15 +442,8 @@ class SymmetricTensor:
         if common.size > 1:
             offsets[1:] = np.cumsum(sizes[:-1])
         out = dev.empty_f64(int(sizes.sum()))
-        problems = [
-            {
-                "A": self._data, "a_off": self._offsets[a], "a_trans": self._trans,
-                "B": other._data, "b_off": other._offsets[b], "b_trans": other._trans,
-                "C": out, "c_off": offsets[i], "M": M[i], "N": N[i], "K": K[i],
-            }
-            for i, (a, b) in enumerate(zip(i1, i2, strict=True))
-        ]
-        linalg.grouped_gemm(problems)
+        linalg.block_gemm(self._data, self._offsets[i1], self._trans, other._data,
+                          other._offsets[i2], other._trans, out, offsets, M, N, K)
         signature = np.empty((self._nrr + other._ndim - other._nrr,), dtype=bool)
         signature[: self._nrr] = self._signature[: self._nrr]
         signature[self._nrr :] = other._signature[other._nrr :]

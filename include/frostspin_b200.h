@@ -259,6 +259,22 @@ int fs_grouped_dgemm_thin(const FsGemmProblem* d_problems, int64_t n_problems,
                           const FsGemmTile* d_tiles, int64_t n_tiles, void* stream);
 
 /*
+ * The same launches for up to FS_DGEMM_LIST_MAX problems given as a HOST array,
+ * which travels with the kernel's parameters: no table copies, no tile list.
+ * Tiles run problem by problem in the given order (column-major in problems
+ * with more tile columns than rows).  kind: FS_DGEMM_TILES as fs_grouped_dgemm,
+ * FS_DGEMM_UNIFORM as fs_grouped_dgemm_uniform (with the flags of the first
+ * problem, which all must share), FS_DGEMM_THIN as fs_grouped_dgemm_thin (every
+ * problem within its limits).
+ */
+#define FS_DGEMM_TILES 0
+#define FS_DGEMM_UNIFORM 1
+#define FS_DGEMM_THIN 2
+#define FS_DGEMM_LIST_MAX 360
+int fs_grouped_dgemm_list(const FsGemmProblem* h_problems, int64_t n_problems, int32_t kind,
+                          void* stream);
+
+/*
  * Split-K completion: C = alpha * sum_{j < nslices} W[j * slice ...] + beta * C
  * for M x N row-major results (C leading dimension ldc, slices contiguous
  * M x N), summed in slice order.  The host cuts a long-K sector problem into
@@ -278,6 +294,10 @@ typedef struct FsSplitReduce {
 
 int fs_splitk_reduce(const FsSplitReduce* d_items, int64_t n_items, int64_t max_elems,
                      void* stream);
+/* The same for a HOST array of at most FS_SPLIT_LIST_MAX items. */
+#define FS_SPLIT_LIST_MAX 48
+int fs_splitk_reduce_list(const FsSplitReduce* h_items, int64_t n_items, int64_t max_elems,
+                          void* stream);
 
 /*
  * Tile table of a grouped GEMM launch, written on the device (a planning
@@ -544,6 +564,13 @@ int fs_weighted_sum(const double* d_x, const FsSegment* d_segs, int64_t n_segs,
                     double* d_partial, int64_t n_partial, double* d_out,
                     void* stream);
 
+/* Both for a HOST array of at most FS_LIST_MAX segments, which travels with the
+ * kernel's parameters; squares != 0: fs_weighted_sumsq. */
+#define FS_LIST_MAX 96
+int fs_weighted_sum_list(const double* d_x, const FsSegment* h_segs, int64_t n_segs,
+                         int32_t squares, double* d_partial, int64_t n_partial, double* d_out,
+                         void* stream);
+
 /*
  * Pairwise block contraction: out[0] = sum_p weight_p * sum_{ij} A_p[i,j] B_p[j,i]
  * (full_contract, symmetric_tensor.py:639-653) or, with b == NULL entries,
@@ -561,6 +588,11 @@ int fs_pair_contract(const double* d_a, const double* d_b,
                      const FsPairBlock* d_pairs, int64_t n_pairs,
                      double* d_partial, int64_t n_partial, double* d_out,
                      void* stream);
+/* The same for a HOST array of at most FS_LIST_MAX pairs. */
+int fs_pair_contract_list(const double* d_a, const double* d_b,
+                          const FsPairBlock* h_pairs, int64_t n_pairs,
+                          double* d_partial, int64_t n_partial, double* d_out,
+                          void* stream);
 
 /*
  * Diagonal scaling of blocks by 1-D weight vectors: out_b[i,j] = x_b[i,j] * d[j]
@@ -575,6 +607,9 @@ typedef struct FsDiagBlock {
 
 int fs_diag_mul(const double* d_x, const double* d_diag, double* d_out,
                 const FsDiagBlock* d_blocks, int64_t n_blocks, void* stream);
+/* The same for a HOST array of at most FS_LIST_MAX blocks. */
+int fs_diag_mul_list(const double* d_x, const double* d_diag, double* d_out,
+                     const FsDiagBlock* h_blocks, int64_t n_blocks, void* stream);
 
 /* Elementwise power of a weight vector, y = x^p, with p = -1, -0.5, 0.5 and
  * 2 exact special cases (DiagonalTensor.__pow__, diagonal_tensor.py:133-143). */
