@@ -279,6 +279,8 @@ SIGNATURES = {
     "fs_grouped_dgemm_thin": (ctypes.c_int, [_P, _I64, _P, _I64, _P]),
     "fs_grouped_dgemm_uniform": (ctypes.c_int, [_P, _I64, _P, _I64, _I32, _I32, _P]),
     "fs_grouped_dgemm_list": (ctypes.c_int, [_P, _I64, _I32, _P]),
+    "fs_dgemm_wide_limits": (ctypes.c_int, [_P, _P, _P]),
+    "fs_grouped_dgemm_wide": (ctypes.c_int, [_P, _I64, _P]),
     "fs_splitk_reduce": (ctypes.c_int, [_P, _I64, _I64, _P]),
     "fs_splitk_reduce_list": (ctypes.c_int, [_P, _I64, _I64, _P]),
     "fs_expand_tiles": (ctypes.c_int, [_P, _I64, _I64, _P, _P]),
@@ -351,7 +353,7 @@ CALL_COUNTS = {}
 LAUNCHES_PER_CALL = {
     "fs_abelian_permute": 1, "fs_abelian_permute_multi": 1,
     "fs_permute_tiles": 1, "fs_permute_tiles_multi": 1, "fs_su2_permute_fused": 1, "fs_grouped_dgemm": 1, "fs_grouped_dgemm_thin": 1,
-    "fs_grouped_dgemm_uniform": 1, "fs_splitk_reduce": 1, "fs_expand_tiles": 1, "fs_ozaki_split": 2,
+    "fs_grouped_dgemm_uniform": 1, "fs_grouped_dgemm_wide": 1, "fs_splitk_reduce": 1, "fs_expand_tiles": 1, "fs_ozaki_split": 2,
     "fs_ozaki_gemm": 1, "fs_ozaki_gemm_pair": 1, "fs_ozaki2_split": 2, "fs_ozaki2_gemm_pair": 1,
     "fs_scale": 1, "fs_scale_by": 1, "fs_axpby": 1, "fs_pow": 1, "fs_weighted_sumsq": 2,
     "fs_weighted_sum": 2, "fs_pair_contract": 2, "fs_diag_mul": 1, "fs_o2_recombine": 1,
@@ -390,6 +392,14 @@ def thin_dgemm_shape():
     tn = ctypes.c_int32()
     call("fs_thin_dgemm_shape", ctypes.byref(mm), ctypes.byref(mk), ctypes.byref(tn))
     return mm.value, mk.value, tn.value
+
+
+def dgemm_wide_limits():
+    a = ctypes.c_int32()
+    b = ctypes.c_int32()
+    c = ctypes.c_int32()
+    call("fs_dgemm_wide_limits", ctypes.byref(a), ctypes.byref(b), ctypes.byref(c))
+    return a.value, b.value, c.value
 
 
 def ozaki2_bits(nmod, K):

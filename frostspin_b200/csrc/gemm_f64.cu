@@ -436,6 +436,281 @@ extern "C" int fs_grouped_dgemm_uniform(const FsGemmProblem* d_problems, int64_t
                          trans_b != 0, fsb::as_stream(stream));
 }
 
+// ---------------------------------------------------------------- wide GEMMs
+// Products of a small matrix with many columns (a corner on a wide half network,
+// projector applications: M and K of a few tens, N of 1e5 and more).  Both the
+// FP64 tensor pipe (2 M K per column) and HBM (8 (M + K) bytes per column) bound
+// them, so neither may wait for the other: op(A) of a problem stays in shared
+// memory for all its columns, and the 16 warps of the SM work on their own strips
+// of 8 NT columns without a CTA barrier.  A warp loads its strip straight into
+// DMMA B fragments (all K rows in flight, four rows of 64 bytes per load),
+// multiplies it by every 8-row block of A, and turns each 8 x 8 NT block of C
+// through a small buffer into whole 64 NT-byte runs.  The 64 x 64 tiles of the
+// streaming kernel reload A for every tile by 8-byte cp.async and write C in
+// halves of sectors.  9 sectors with M = K = 7 to 51 and N = 0.1 to 0.2 M: 313 us
+// there (L2 write sectors 4 times the ideal), 201 us here.
+//
+// CTA b takes an equal share of the estimated time of all strips, problem by
+// problem, so it loads one or two A.
+namespace fsb {
+
+constexpr int kWideWarps = 16;
+constexpr int kWideThreads = 32 * kWideWarps;
+constexpr int kWideMaxProblems = 40;
+constexpr int kWideBufC = 16 * (16 + 2);   // a warp's block of C
+// doubles of the largest op(A) beside the C buffers, in 227 KB
+constexpr int kWideMaxA = 227 * 1024 / 8 - kWideWarps * kWideBufC;
+
+struct WideList {
+    FsGemmProblem v[kWideMaxProblems];
+    int32_t n_problems;
+    int32_t a_doubles;   // shared doubles of the largest op(A)
+};
+
+// padded rows, k and leading dimension of A in shared memory: 4 mod 8 doubles,
+// so that the 8 x 4 fragment reads of a half warp touch distinct banks
+__host__ __device__ __forceinline__ int wide_rows(int M) { return (M + 7) / 8 * 8; }
+// k steps of 4, rounded up to an instantiated number
+__host__ __device__ __forceinline__ int wide_steps(int K) {
+    const int n = K > 4 ? (K + 3) / 4 : 1;
+    return n <= 2 ? n : (n + 1) / 2 * 2;
+}
+__host__ __device__ __forceinline__ int wide_k(int K) { return 4 * wide_steps(K); }
+__host__ __device__ __forceinline__ int wide_ld(int K) {
+    const int k4 = wide_k(K);
+    return k4 % 8 == 0 ? k4 + 4 : k4;
+}
+// columns of a strip: its fragments take up to 64 registers, and longer runs of B
+// and C rows serve short K (M = K = 8 on 2 M columns 50 us in strips of 32, 64 us
+// in strips of 16; M = K = 32 on 0.6 M columns 87 and 72 us)
+__host__ __device__ __forceinline__ int wide_cols(int K) {
+    return wide_steps(K) <= 4 ? 32 : wide_steps(K) <= 16 ? 16 : 8;
+}
+// relative time of a strip: FP64 FMAs at 64 per cycle and SM, bytes at 23; the
+// shorter of the two is about half hidden
+__host__ __device__ __forceinline__ int64_t wide_cost(int M, int K) {
+    const int64_t math = static_cast<int64_t>(wide_rows(M)) * wide_k(K) / 64;
+    const int64_t mem = static_cast<int64_t>(M + K) * 8 / 23;
+    return (math > mem ? 2 * math + mem : 2 * mem + math) * wide_cols(K) + 1;
+}
+
+// The columns n0 .. n0 + 8 NT - 1 of op(B) as DMMA fragments, one k step at a
+// time; columns past `left` and rows past K are zero.
+struct WideSource {
+    const double* p;   // this lane's row of step 0, column 0
+    int64_t sk, sn;
+    int K, left;       // columns left, 0: nothing to load
+    template <int NT>
+    __device__ __forceinline__ void load(double (&b)[NT], int ks) {
+        const int lane = threadIdx.x % 32;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const bool ok = 4 * ks + (lane & 3) < K && 8 * j + (lane >> 2) < left;
+            b[j] = ok ? __ldg(p + 8 * j * sn) : 0.0;
+        }
+        p += 4 * sk;
+    }
+};
+
+// H blocks of 8 rows of C = A b for one strip: A at pa (this lane's fragment
+// row and k), through the warp's buffer sc to d, `rows` rows left.  kNext: the
+// strip's last rows; each fragment of b is replaced by the next strip's once its
+// products are issued, so that the loads run behind the products and the stores.
+template <int H, bool kNext, int NT, int KS>
+__device__ __forceinline__ void wide_rows_of(double (&b)[KS][NT], const double* pa, int ld,
+                                             double* sc, double* d, int64_t ldc, int rows,
+                                             bool col_ok, double alpha, double beta,
+                                             WideSource next) {
+    constexpr int kCols = 8 * NT;
+    constexpr int kLdC = kCols + 2;
+    const int lane = threadIdx.x % 32;
+    const int fr = lane >> 2, fk = lane & 3;
+    double acc[H][NT][2];
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[h][j][0] = acc[h][j][1] = 0.0;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const double a = pa[h * 8 * ld + 4 * ks];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) dmma(acc[h][j], a, b[ks][j]);
+        }
+        if (kNext) next.load(b[ks], ks);
+    }
+    __syncwarp();   // the previous block has been stored
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+            *reinterpret_cast<double2*>(sc + (8 * h + fr) * kLdC + 8 * j + 2 * fk) =
+                make_double2(alpha * acc[h][j][0], alpha * acc[h][j][1]);
+    __syncwarp();
+    const int r0 = lane / kCols;
+    const double* c = sc + r0 * kLdC + lane % kCols;
+    if (!col_ok) return;
+    if (beta == 0.0) {
+#pragma unroll
+        for (int r = 0; r < 8 * H; r += 32 / kCols) {
+            if (r + r0 < rows) *d = c[r * kLdC];
+            d += (32 / kCols) * ldc;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < 8 * H; r += 32 / kCols) {
+            if (r + r0 < rows) *d = fma(beta, *d, c[r * kLdC]);
+            d += (32 / kCols) * ldc;
+        }
+    }
+}
+
+// The strips [first, last) of one problem, k steps padded to KS with zeros, H
+// blocks of 8 rows at a time.
+template <int H, int NT, int KS>
+__device__ __forceinline__ void wide_strips(const FsGemmProblem& p, const double* sa, int ld,
+                                            double* sc, int64_t first, int64_t last) {
+    constexpr int kCols = 8 * NT;
+    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+    const int fr = lane >> 2, fk = lane & 3;
+    const int M = p.M, N = p.N, K = p.K;
+    const int64_t sk = p.transB ? 1 : p.ldb, sn = p.transB ? p.ldb : 1;
+    const int64_t ldc = p.ldc;
+    const double alpha = p.alpha, beta = p.beta;
+    const double* pa = sa + fr * ld + fk;
+    auto source = [&](int64_t strip) {
+        const int64_t n0 = strip * kCols;
+        return WideSource{p.B + fk * sk + (n0 + fr) * sn, sk, sn, K,
+                          strip < last ? static_cast<int>(min(N - n0, static_cast<int64_t>(kCols)))
+                                       : 0};
+    };
+    int64_t s = first + wid;
+    double b[KS][NT];
+    WideSource now = source(s);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) now.load(b[ks], ks);
+#pragma unroll 1
+    for (; s < last; s += kWideWarps) {
+        const int64_t n0 = s * kCols;
+        const WideSource next = source(s + kWideWarps);
+        const bool col_ok = n0 + lane % kCols < N;
+        double* d = p.C + (lane / kCols) * ldc + n0 + lane % kCols;
+        int m0 = 0;
+#pragma unroll 1
+        for (; m0 + 8 * H < M; m0 += 8 * H) {
+            wide_rows_of<H, false>(b, pa + m0 * ld, ld, sc, d, ldc, 8 * H, col_ok, alpha, beta,
+                                   next);
+            d += 8 * H * ldc;
+        }
+        if (H > 1 && m0 + 8 < M)
+            wide_rows_of<H, true>(b, pa + m0 * ld, ld, sc, d, ldc, M - m0, col_ok, alpha, beta,
+                                  next);
+        else
+            wide_rows_of<1, true>(b, pa + m0 * ld, ld, sc, d, ldc, M - m0, col_ok, alpha, beta,
+                                  next);
+    }
+}
+
+__global__ void __launch_bounds__(kWideThreads, 1)
+    k_dgemm_wide(const __grid_constant__ WideList list) {
+    extern __shared__ __align__(16) double wide_smem[];
+    double* sa = wide_smem;
+    double* sc = wide_smem + list.a_doubles + threadIdx.x / 32 * kWideBufC;
+
+    int64_t total = 0;
+    for (int i = 0; i < list.n_problems; ++i) {
+        const FsGemmProblem& p = list.v[i];
+        const int cols = wide_cols(p.K);
+        total += static_cast<int64_t>((p.N + cols - 1) / cols) * wide_cost(p.M, p.K);
+    }
+    const int64_t lo = total / gridDim.x * blockIdx.x +
+                       total % gridDim.x * blockIdx.x / gridDim.x;
+    const int64_t hi = total / gridDim.x * (blockIdx.x + 1) +
+                       total % gridDim.x * (blockIdx.x + 1) / gridDim.x;
+    int64_t pos = 0;
+#pragma unroll 1
+    for (int i = 0; i < list.n_problems && pos < hi; ++i) {
+        const FsGemmProblem& p = list.v[i];
+        const int64_t cost = wide_cost(p.M, p.K);
+        const int cols = wide_cols(p.K);
+        const int64_t strips = (p.N + cols - 1) / cols;
+        const int64_t first = lo > pos ? (lo - pos + cost - 1) / cost : 0;
+        const int64_t last = min((hi - pos + cost - 1) / cost, strips);
+        pos += strips * cost;
+        if (first >= last || p.M <= 0) continue;
+        const int m8 = wide_rows(p.M), k4 = wide_k(p.K), ld = wide_ld(p.K);
+        __syncthreads();   // the previous problem's A has been read
+        for (int e = threadIdx.x; e < m8 * k4; e += kWideThreads) {
+            // consecutive threads along the contiguous direction of A
+            const int m = p.transA ? e % m8 : e / k4, k = p.transA ? e / m8 : e % k4;
+            double v = 0.0;
+            if (m < p.M && k < p.K)
+                v = p.A[p.transA ? static_cast<int64_t>(k) * p.lda + m
+                                 : static_cast<int64_t>(m) * p.lda + k];
+            sa[m * ld + k] = v;
+        }
+        __syncthreads();
+        switch (k4 / 4) {
+#define FSB_WIDE(h, nt, ks) \
+    case ks: wide_strips<h, nt, ks>(p, sa, ld, sc, first, last); break;
+            FSB_WIDE(1, 4, 1)
+            FSB_WIDE(1, 4, 2)
+            FSB_WIDE(1, 4, 4)
+            FSB_WIDE(2, 2, 6)
+            FSB_WIDE(2, 2, 8)
+            FSB_WIDE(2, 2, 10)
+            FSB_WIDE(2, 2, 12)
+            FSB_WIDE(2, 2, 14)
+            FSB_WIDE(2, 2, 16)
+            FSB_WIDE(2, 1, 18)
+            FSB_WIDE(2, 1, 20)
+            FSB_WIDE(2, 1, 22)
+            FSB_WIDE(2, 1, 24)
+            FSB_WIDE(2, 1, 26)
+            FSB_WIDE(2, 1, 28)
+            FSB_WIDE(2, 1, 30)
+            FSB_WIDE(2, 1, 32)
+#undef FSB_WIDE
+        }
+    }
+}
+
+}  // namespace fsb
+
+extern "C" int fs_dgemm_wide_limits(int32_t* max_problems, int32_t* max_k, int32_t* max_a) {
+    if (max_problems == nullptr || max_k == nullptr || max_a == nullptr) return FS_ERR_INVALID_ARG;
+    *max_problems = fsb::kWideMaxProblems;
+    *max_k = 128;
+    *max_a = fsb::kWideMaxA;
+    return FS_OK;
+}
+
+extern "C" int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_problems,
+                                     void* stream) {
+    if (n_problems < 0) return FS_ERR_INVALID_ARG;
+    if (n_problems == 0) return FS_OK;
+    if (h_problems == nullptr) return FS_ERR_INVALID_ARG;
+    if (n_problems > fsb::kWideMaxProblems) return FS_ERR_TOO_LARGE;
+    fsb::WideList list;
+    memcpy(list.v, h_problems, sizeof(FsGemmProblem) * static_cast<size_t>(n_problems));
+    list.n_problems = static_cast<int32_t>(n_problems);
+    list.a_doubles = 0;
+    for (int64_t i = 0; i < n_problems; ++i) {
+        const FsGemmProblem& p = h_problems[i];
+        if (p.M < 0 || p.N < 0 || p.K < 0) return FS_ERR_INVALID_ARG;
+        const int64_t a = static_cast<int64_t>(fsb::wide_rows(p.M)) * fsb::wide_ld(p.K);
+        if (p.K > 128 || a > fsb::kWideMaxA) return FS_ERR_TOO_LARGE;
+        if (a > list.a_doubles) list.a_doubles = static_cast<int32_t>(a);
+    }
+    const int bytes = static_cast<int>(sizeof(double)) *
+                      (list.a_doubles + fsb::kWideWarps * fsb::kWideBufC);
+    const int st = fsb::configure_smem(reinterpret_cast<const void*>(fsb::k_dgemm_wide), bytes);
+    if (st != FS_OK) return st;
+    fsb::k_dgemm_wide<<<fsb::num_sms(), fsb::kWideThreads, bytes, fsb::as_stream(stream)>>>(list);
+    return fsb::launch_status();
+}
+
 // ---------------------------------------------------------------- thin GEMMs
 // C[MxN] = alpha A[MxK] B[KxN] + beta C for M, K <= 32 and N large: the
 // recoupling products of a non-abelian permute (one small isometry applied to

@@ -502,6 +502,26 @@ def _tile_counts(arr, tm, tn):
 _STREAM_MAX_K = 256   # longest K of a launch that goes to the streaming kernel
 
 
+_WIDE = {}
+_WIDE_COLUMNS = 148 * 16 * 16 * 2   # two strips of 16 columns for every warp
+
+
+def _wide(arr):
+    """Whether a launch goes to the wide kernel: op(A) of every problem in shared
+    memory, and columns enough for all its warps."""
+    if not _WIDE:
+        _WIDE["limits"] = _native.dgemm_wide_limits()
+    max_n, max_k, max_a = _WIDE["limits"]
+    if arr.size > max_n or int(arr["K"].max()) > max_k:
+        return False
+    N = arr["N"].astype(np.int64)
+    if int(N.sum()) < _WIDE_COLUMNS:
+        return False
+    # rows in eights, k steps of 4 in pairs, and 4 doubles against bank conflicts
+    a = _pad(arr["M"].astype(np.int64), 8) * (_pad(arr["K"].astype(np.int64), 8) + 4)
+    return int(a.max()) <= max_a
+
+
 # The tables cost the host about 60 us and the device 8 us, hidden once a launch
 # runs longer than that; the per-tile kernel itself is 0.6 % faster with them
 # (10 335 tiles of K up to 2900: 6.81 ms with tables, 6.86 by value; 1008 tiles
@@ -526,6 +546,10 @@ def _launch_dgemm(arr):
     FS_DGEMM_LIST_MAX problems travel with the launch; longer tables, and
     launches of the per-tile kernel beyond _LIST_TILES tiles, go through device
     memory with their tile list."""
+    if _wide(arr):
+        arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
+        _native.call("fs_grouped_dgemm_wide", arr.ctypes.data, arr.size, dev.stream())
+        return
     ta, tb = arr["transA"], arr["transB"]
     uniform = ((ta == ta[0]).all() and (tb == tb[0]).all()
                and int(arr["K"].max()) <= _STREAM_MAX_K)

@@ -275,6 +275,15 @@ int fs_grouped_dgemm_list(const FsGemmProblem* h_problems, int64_t n_problems, i
                           void* stream);
 
 /*
+ * The same products for small matrices on many columns: op(A) of each problem
+ * stays in shared memory (padded M x K at most max_a doubles, K <= max_k), the
+ * warps stream the columns.  At most max_problems problems, a HOST array, any
+ * transpose flags.  Same call sites as fs_grouped_dgemm.
+ */
+int fs_dgemm_wide_limits(int32_t* max_problems, int32_t* max_k, int32_t* max_a);
+int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_problems, void* stream);
+
+/*
  * Split-K completion: C = alpha * sum_{j < nslices} W[j * slice ...] + beta * C
  * for M x N row-major results (C leading dimension ldc, slices contiguous
  * M x N), summed in slice order.  The host cuts a long-K sector problem into
