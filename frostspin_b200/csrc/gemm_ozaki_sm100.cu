@@ -1105,95 +1105,106 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 // any half integer) and the residue is the low byte of A' - q p computed in
 // 32-bit integers.  For p = 256 it is the low byte of A'.
 //
-// Thread mapping: a block handles a 32-row group of one k-tile (32 rows x 128
-// k values); each thread 16 consecutive k of one row.  When the operand's rows
-// are contiguous in memory (transposed storage) a warp spans 32 rows at one
-// k-chunk and reads them directly, coalesced.  Otherwise (k contiguous) the
-// block first copies the 32 x 128 tile into shared memory with consecutive
-// threads on consecutive k (a thread's own 16 k would spread one warp load over
-// 32 sectors), each 16-value chunk padded to 17 doubles so that the threads of
-// a half warp read 16 distinct bank pairs.
-constexpr int kSplitPad = 17;
+// A block handles a 32-row group of one k-tile (32 rows x 128 k values).  It
+// first copies the tile into shared memory with consecutive threads along the
+// operand's contiguous direction; then 16 threads take one row, 8 consecutive k
+// each, for two rows in turn, so that the 8-byte stores of a warp fill whole
+// 128-byte rows of every slice.  Each 8-value chunk is padded to 9 doubles and
+// each row to 145: both the copies (along k or along rows) and the reads touch
+// distinct banks.
+//
+// Bound by issue slots and HBM (8 bytes read and n written per entry): the
+// residues cost one FP64 FMA and one integer multiply-add per entry and modulus,
+// packed four to a word by byte permutes.  Two operands of 114 M entries, 11
+// moduli: 1991 us with 16 k per thread, whose stores filled 8 of every 16 bytes
+// at a time, and shifts and masks for the packing; 796 us now (5.4 TB/s; with 3
+// or 5 CTAs per SM 889 and 837 us).
+constexpr int kSplitChunk = 9;                    // 8 k and one double of padding
+constexpr int kSplitLd = 16 * kSplitChunk + 1;    // a row of the staged tile
 
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, 4)
     k_oz2_split(const FsOz2Operand* __restrict__ ops, int64_t n_ops,
                 const __grid_constant__ CrtConsts cc) {
-    __shared__ double stage[32 * 8 * kSplitPad];
+    __shared__ double stage[32 * kSplitLd];
     const int op_id = blockIdx.y;
     if (op_id >= n_ops) return;
     const FsOz2Operand op = ops[op_id];
     const bool rows_contiguous = (op.s_row == 1 && op.s_k != 1);
     const int t = threadIdx.x;
-    const int r = rows_contiguous ? (t & 31) : (t >> 3);   // row within the 32-row group
-    const int c = rows_contiguous ? (t >> 5) : (t & 7);    // 16-byte chunk of the k-tile
+    const int hc = t % 16;
     const int groups = op.rowtiles * (kSplitRows / 32);
     const int64_t units = static_cast<int64_t>(groups) * op.ktiles;
     const int64_t slice_stride = static_cast<int64_t>(op.ktiles) * op.rowtiles * kABytes;
     const int n = cc.n;
     for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
         const int kt = static_cast<int>(u / groups);
-        const int rg = static_cast<int>(u % groups);
+        const int rg = static_cast<int>(u - static_cast<int64_t>(kt) * groups);
         const int rt = rg / (kSplitRows / 32);
-        const int rr = (rg % (kSplitRows / 32)) * 32 + r;       // row within the tile
-        const int64_t row = static_cast<int64_t>(rt) * kSplitRows + rr;
-        const int64_t k0 = static_cast<int64_t>(kt) * kTileK + c * 16;
-        const bool row_ok = row < op.rows;
-        const int sh = op.bits - (row_ok ? op.exps[row] : 0);
-        if (!rows_contiguous) {
-            // coalesced copy of the block's 32 rows x 128 k into shared memory
-            const int64_t row_base = static_cast<int64_t>(rt) * kSplitRows +
-                                     (rg % (kSplitRows / 32)) * 32;
-            const int64_t kb = static_cast<int64_t>(kt) * kTileK;
-            __syncthreads();   // the previous unit's reads of the stage are done
+        const int r0 = (rg % (kSplitRows / 32)) * 32;           // first row within the tile
+        const int64_t row_base = static_cast<int64_t>(rt) * kSplitRows + r0;
+        const int rows = static_cast<int>(min(static_cast<int64_t>(32), op.rows - row_base));
+        const int ks = static_cast<int>(min(static_cast<int64_t>(kTileK),
+                                            op.K - static_cast<int64_t>(kt) * kTileK));
+        __syncthreads();   // the previous unit's reads of the stage are done
+        {
+            // thread t copies 16 entries: k = t % 128 of every second row, or
+            // row t % 32 at every eighth k
+            const int sr = rows_contiguous ? t % 32 : t / 128;
+            const int sk = rows_contiguous ? t / 32 : t % 128;
+            const double* src = op.src + (row_base + sr) * op.s_row +
+                                (static_cast<int64_t>(kt) * kTileK + sk) * op.s_k;
+            const int64_t step = rows_contiguous ? 8 * op.s_k : 2 * op.s_row;
+            double v[16];
 #pragma unroll
             for (int it = 0; it < 16; ++it) {
-                const int e = it * 256 + t;
-                const int sr = e >> 7, sk = e & 127;
-                const int64_t grow = row_base + sr, gk = kb + sk;
-                stage[(sr * 8 + (sk >> 4)) * kSplitPad + (sk & 15)] =
-                    (grow < op.rows && gk < op.K) ? __ldg(op.src + grow * op.s_row + gk * op.s_k)
-                                                  : 0.0;
+                const bool ok = rows_contiguous ? sr < rows && sk + 8 * it < ks
+                                                : sr + 2 * it < rows && sk < ks;
+                v[it] = ok ? __ldg(src) : 0.0;
+                src += step;
             }
-            __syncthreads();
-        }
-        int8_t* dst = op.slices + (static_cast<int64_t>(kt) * op.rowtiles + rt) * kABytes +
-                      rr * 128 + ((c ^ (rr & 7)) * 16);
-        // the 16 k of this thread in two halves of 8 (8-byte stores per
-        // modulus): half the live operand registers, so that three CTAs fit on
-        // an SM without spills
+            double* d = stage + sr * kSplitLd + (sk / 8) * kSplitChunk + sk % 8;
+            const int dstep = rows_contiguous ? kSplitChunk : 2 * kSplitLd;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            int32_t lo[8];
+            for (int it = 0; it < 16; ++it) {
+                *d = v[it];
+                d += dstep;
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+            const int r = t / 16 + 16 * pass, rr = r0 + r;
+            const int sh = op.bits - (r < rows ? op.exps[row_base + r] : 0);
+            int8_t* dst = op.slices + (static_cast<int64_t>(kt) * op.rowtiles + rt) * kABytes +
+                          rr * 128 + (((hc >> 1) ^ (rr & 7)) * 16) + (hc & 1) * 8;
+            const double* x = stage + r * kSplitLd + hc * kSplitChunk;
+            uint32_t lo[8];
             double ad[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int64_t k = k0 + 8 * h + j;
-                double x;
-                if (rows_contiguous)
-                    x = (row_ok && k < op.K) ? __ldg(op.src + row * op.s_row + k * op.s_k) : 0.0;
-                else
-                    x = stage[(r * 8 + c) * kSplitPad + 8 * h + j];
-                const double tt = scale2(x, sh) + kRoundMagic;
-                lo[j] = __double2loint(tt);
+                const double tt = scale2(x[j], sh) + kRoundMagic;
+                lo[j] = static_cast<uint32_t>(__double2loint(tt));
                 ad[j] = tt - kRoundMagic;
             }
-            {
-                uint32_t w[2] = {0, 0};
+            auto store = [&](int8_t* d, const uint32_t (&v)[8]) {
+                const uint32_t w0 = __byte_perm(__byte_perm(v[0], v[1], 0x0040),
+                                                __byte_perm(v[2], v[3], 0x0040), 0x5410);
+                const uint32_t w1 = __byte_perm(__byte_perm(v[4], v[5], 0x0040),
+                                                __byte_perm(v[6], v[7], 0x0040), 0x5410);
+                *reinterpret_cast<uint2*>(d) = make_uint2(w0, w1);
+            };
+            store(dst, lo);
+#pragma unroll 2
+            for (int m = 1; m < n; ++m) {
+                const uint32_t pm = static_cast<uint32_t>(cc.p[m]);
+                const double ipm = cc.inv_p[m];
+                uint32_t v[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    w[j / 4] |= (static_cast<uint32_t>(lo[j]) & 0xFFu) << (8 * (j % 4));
-                *reinterpret_cast<uint2*>(dst + 8 * h) = make_uint2(w[0], w[1]);
-            }
-            for (int m = 1; m < n; ++m) {
-                const int32_t pm = cc.p[m];
-                const double ipm = cc.inv_p[m];
-                uint32_t w[2] = {0, 0};
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int32_t q = __double2loint(fma(ad[j], ipm, kRoundMagic));
-                    w[j / 4] |= (static_cast<uint32_t>(lo[j] - q * pm) & 0xFFu) << (8 * (j % 4));
-                }
-                *reinterpret_cast<uint2*>(dst + m * slice_stride + 8 * h) = make_uint2(w[0], w[1]);
+                    v[j] = lo[j] - static_cast<uint32_t>(__double2loint(
+                                       fma(ad[j], ipm, kRoundMagic))) * pm;
+                dst += slice_stride;
+                store(dst, v);
             }
         }
     }
