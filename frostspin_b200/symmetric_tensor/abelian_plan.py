@@ -51,9 +51,14 @@ def segments(rep):
 
 
 def _cyclic_conv(h, s):
-    c = np.arange(256)
-    idx = (c[:, None] - c[None, :]) % 256
-    return (h[None, :] * s[idx]).sum(axis=1)
+    """Counts of charge sums modulo 256: out[c] = sum_a h[a] s[c - a].  A leg
+    carries a few charges, so only the shifts that occur are added (the full
+    256 x 256 product took 330 us, three quarters of a block-size query)."""
+    out = np.zeros(256, dtype=np.int64)
+    twice = np.concatenate([s, s])
+    for a in np.flatnonzero(h):
+        out += h[a] * twice[256 - a : 512 - a]
+    return out
 
 
 class GroupInfo:
