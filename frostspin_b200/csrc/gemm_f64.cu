@@ -215,7 +215,7 @@ struct TileList {
     };
     template <int TM, int TN>
     __host__ __device__ __forceinline__ static int64_t count(const FsGemmProblem& p) {
-        return static_cast<int64_t>((p.M + TM - 1) / TM) * ((p.N + TN - 1) / TN);
+        return (static_cast<int64_t>(p.M) + TM - 1) / TM * ((static_cast<int64_t>(p.N) + TN - 1) / TN);
     }
     template <int TM, int TN>
     __device__ __forceinline__ bool find(Cursor& c, int64_t t, FsGemmProblem& p, int& m0,
@@ -231,7 +231,8 @@ struct TileList {
         asm volatile("" : "+l"(p.A), "+l"(p.B), "+l"(p.lda), "+l"(p.ldb), "+r"(p.M), "+r"(p.N), "+r"(p.K));
         // a problem has fewer than 2^31 tiles (host)
         const uint32_t k = static_cast<uint32_t>(t - c.first);
-        const uint32_t nr = (p.M + TM - 1) / TM, nc = (p.N + TN - 1) / TN;
+        const uint32_t nr = (static_cast<uint32_t>(p.M) + TM - 1) / TM;
+        const uint32_t nc = (static_cast<uint32_t>(p.N) + TN - 1) / TN;
         const uint32_t q = k / (nc > nr ? nr : nc), r = k - q * (nc > nr ? nr : nc);
         m0 = static_cast<int>(nc > nr ? r : q) * TM;
         n0 = static_cast<int>(nc > nr ? q : r) * TN;
@@ -622,7 +623,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     for (int i = 0; i < list.n_problems; ++i) {
         const FsGemmProblem& p = list.v[i];
         const int cols = wide_cols(p.K);
-        total += static_cast<int64_t>((p.N + cols - 1) / cols) * wide_cost(p.M, p.K);
+        total += (static_cast<int64_t>(p.N) + cols - 1) / cols * wide_cost(p.M, p.K);
     }
     const int64_t lo = total / gridDim.x * blockIdx.x +
                        total % gridDim.x * blockIdx.x / gridDim.x;
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         const FsGemmProblem& p = list.v[i];
         const int64_t cost = wide_cost(p.M, p.K);
         const int cols = wide_cols(p.K);
-        const int64_t strips = (p.N + cols - 1) / cols;
+        const int64_t strips = (static_cast<int64_t>(p.N) + cols - 1) / cols;
         const int64_t first = lo > pos ? (lo - pos + cost - 1) / cost : 0;
         const int64_t last = min((hi - pos + cost - 1) / cost, strips);
         pos += strips * cost;
@@ -699,8 +700,9 @@ extern "C" int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_
     for (int64_t i = 0; i < n_problems; ++i) {
         const FsGemmProblem& p = h_problems[i];
         if (p.M < 0 || p.N < 0 || p.K < 0) return FS_ERR_INVALID_ARG;
+        if (p.K > 128 || p.M > fsb::kWideMaxA) return FS_ERR_TOO_LARGE;
         const int64_t a = static_cast<int64_t>(fsb::wide_rows(p.M)) * fsb::wide_ld(p.K);
-        if (p.K > 128 || a > fsb::kWideMaxA) return FS_ERR_TOO_LARGE;
+        if (a > fsb::kWideMaxA) return FS_ERR_TOO_LARGE;
         if (a > list.a_doubles) list.a_doubles = static_cast<int32_t>(a);
     }
     const int bytes = static_cast<int>(sizeof(double)) *
