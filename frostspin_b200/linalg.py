@@ -514,26 +514,27 @@ def _wide(arr):
     max_n, max_k, max_a = _WIDE["limits"]
     if arr.size > max_n or int(arr["K"].max()) > max_k:
         return False
-    N = arr["N"].astype(np.int64)
-    if int(N.sum()) < _WIDE_COLUMNS:
+    if int(arr["N"].sum()) < _WIDE_COLUMNS:
         return False
     # rows in eights, k steps of 4 in pairs, and 4 doubles against bank conflicts
     a = _pad(arr["M"].astype(np.int64), 8) * (_pad(arr["K"].astype(np.int64), 8) + 4)
     return int(a.max()) <= max_a
 
 
-# The tables cost the host about 60 us and the device 8 us, hidden once a launch
-# runs longer than that; the per-tile kernel itself is 0.6 % faster with them
-# (10 335 tiles of K up to 2900: 6.81 ms with tables, 6.86 by value; 1008 tiles
-# 227 us both).  The streaming kernel is faster by value (wide sectors 313 us,
-# with tables 336 us).
-_LIST_TILES = 4 * 3 * 148
+# The tables cost the host about 100 us (318 recoupling products of an enlarged
+# corner, 141 us of device time: 1020 us a corner with them, 907 by value) and
+# are hidden only behind launches of milliseconds; there the per-tile kernel is
+# 0.6 % faster with them (10 335 tiles, 1.9e11 operations: 6.81 ms with tables,
+# 6.86 by value).  The streaming kernel is always faster by value (wide sectors
+# 313 us, with tables 336 us).
+_TABLE_FLOPS = 1e11
 
 
 def _dgemm_list(name, arr, kind):
     """Launch kernel `name` with the problems passed by value, longest K first
     (long tiles start early in the static schedule)."""
-    arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
+    if arr.size > 1:
+        arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
     _native.call(name, arr.ctypes.data, arr.size, kind, dev.stream(),
                  entry="fs_grouped_dgemm_list")
 
@@ -544,24 +545,23 @@ def _launch_dgemm(arr):
     padded fragments dominate there), else the per-tile kernel (faster on long
     K, where it keeps a few registers more for the DMMA loop).  Up to
     FS_DGEMM_LIST_MAX problems travel with the launch; longer tables, and
-    launches of the per-tile kernel beyond _LIST_TILES tiles, go through device
-    memory with their tile list."""
-    if _wide(arr):
+    launches of the per-tile kernel from _TABLE_FLOPS on, go through device memory
+    with their tile list."""
+    if int(arr["N"].sum()) >= _WIDE_COLUMNS and _wide(arr):
         arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
         _native.call("fs_grouped_dgemm_wide", arr.ctypes.data, arr.size, dev.stream())
         return
     ta, tb = arr["transA"], arr["transB"]
     uniform = ((ta == ta[0]).all() and (tb == tb[0]).all()
                and int(arr["K"].max()) <= _STREAM_MAX_K)
-    tm, tn = _tile_shape()
-    counts = _tile_counts(arr, tm, tn)
-    if arr.size <= _native.FS_DGEMM_LIST_MAX and (uniform or int(counts.sum()) <= _LIST_TILES):
+    if arr.size <= _native.FS_DGEMM_LIST_MAX and (uniform or _flops(arr) < _TABLE_FLOPS):
         if uniform:
             _dgemm_list("fs_grouped_dgemm_uniform", arr, _native.FS_DGEMM_UNIFORM)
         else:
             _dgemm_list("fs_grouped_dgemm", arr, _native.FS_DGEMM_TILES)
         return
-    d_tiles, n_tiles = _tile_table(arr, tm, tn, counts)
+    tm, tn = _tile_shape()
+    d_tiles, n_tiles = _tile_table(arr, tm, tn, _tile_counts(arr, tm, tn))
     d_prob = dev.upload(arr)
     if uniform:
         _native.call("fs_grouped_dgemm_uniform", d_prob.data_ptr(), arr.size,
