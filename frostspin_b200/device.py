@@ -19,7 +19,6 @@ import torch  # noqa: E402
 
 from . import _native  # noqa: E402
 
-_scratch = {}
 _available = []
 _devices = {}
 
@@ -65,15 +64,11 @@ def upload_f64(arr):
     return torch.from_numpy(a).pin_memory().to(device(), non_blocking=True)
 
 
-def scratch_partials():
-    """Per-device scratch for two-pass reductions (fs_reduce_partials() doubles)."""
-    dev = device()
-    key = ("partials", dev.index)
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = torch.empty(_native.reduce_partials(), dtype=torch.float64, device=dev)
-        _scratch[key] = buf
-    return buf
+def reduction_buffer(device):
+    """Memory of one two-pass reduction: its result, then fs_reduce_partials()
+    doubles.  Allocated per call, so that reductions on several streams or
+    threads never share partial sums (torch's allocator orders reuse by stream)."""
+    return torch.empty(1 + _native.reduce_partials(), dtype=torch.float64, device=device)
 
 
 def empty_f64(n):

@@ -884,46 +884,46 @@ def check_ozaki_flags():
 def weighted_reduce(buf, offsets, lengths, weights, *, squares):
     """sum_s w_s sum_i f(buf[off_s + i]) with f = x^2 or x; returns a 0-d device
     tensor (no host synchronisation)."""
-    out = torch.empty(1, dtype=torch.float64, device=buf.device)
+    sums = dev.reduction_buffer(buf.device)
+    out, part, n_part = sums[0], sums.data_ptr() + 8, sums.numel() - 1
     segs = np.zeros(len(offsets), dtype=_native.SEGMENT_DTYPE)
     segs["offset"] = offsets
     segs["length"] = lengths
     segs["weight"] = weights
-    part = dev.scratch_partials()
     name = "fs_weighted_sumsq" if squares else "fs_weighted_sum"
     if segs.size <= _native.FS_LIST_MAX:
         _native.call(name, dev.ptr(buf), segs.ctypes.data, segs.size, int(squares),
-                     part.data_ptr(), part.numel(), out.data_ptr(), dev.stream(),
+                     part, n_part, out.data_ptr(), dev.stream(),
                      entry="fs_weighted_sum_list")
-        return out[0]
+        return out
     d_segs = dev.upload(segs)
     _native.call(
         name,
         dev.ptr(buf),
         d_segs.data_ptr(),
         segs.size,
-        part.data_ptr(),
-        part.numel(),
+        part,
+        n_part,
         out.data_ptr(),
         dev.stream(),
     )
-    return out[0]
+    return out
 
 
 def pair_contract(abuf, bbuf, pairs):
     """pairs: list of (a_off, b_off, m, n, a_trans, b_trans, weight); b_off < 0
     means trace of the A block.  Returns a 0-d device tensor."""
-    out = torch.empty(1, dtype=torch.float64, device=abuf.device)
+    sums = dev.reduction_buffer(abuf.device)
+    out, part, n_part = sums[0], sums.data_ptr() + 8, sums.numel() - 1
     tab = np.zeros(len(pairs), dtype=_native.PAIR_BLOCK_DTYPE)
     if len(pairs):
         tab[:] = [tuple(p) for p in pairs]
-    part = dev.scratch_partials()
     b_ptr = dev.ptr(bbuf) if bbuf is not None else None
     if tab.size <= _native.FS_LIST_MAX:
         _native.call("fs_pair_contract", dev.ptr(abuf), b_ptr, tab.ctypes.data, tab.size,
-                     part.data_ptr(), part.numel(), out.data_ptr(), dev.stream(),
+                     part, n_part, out.data_ptr(), dev.stream(),
                      entry="fs_pair_contract_list")
-        return out[0]
+        return out
     d_tab = dev.upload(tab)
     _native.call(
         "fs_pair_contract",
@@ -931,12 +931,12 @@ def pair_contract(abuf, bbuf, pairs):
         b_ptr,
         d_tab.data_ptr(),
         tab.size,
-        part.data_ptr(),
-        part.numel(),
+        part,
+        n_part,
         out.data_ptr(),
         dev.stream(),
     )
-    return out[0]
+    return out
 
 
 def axpby(x, y, a, b):
