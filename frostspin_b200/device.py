@@ -64,6 +64,46 @@ def upload_f64(arr):
     return torch.from_numpy(a).pin_memory().to(device(), non_blocking=True)
 
 
+class KeptTables:
+    """Device tables uploaded once and used by later calls, whatever their stream.
+    The first call on a stream other than the upload's waits for the upload and
+    marks the tables as used there, so that an evicted plan's memory is not
+    handed on while that stream still reads it.  Inside a graph capture new
+    tables are not kept (their upload runs with the graph) and kept ones are
+    not waited for (an event from outside the capture cannot be)."""
+
+    __slots__ = ("_kept",)
+
+    def __init__(self):
+        self._kept = None
+
+    def get(self, make):
+        """The tables of make() (nested tuples of tensors and None)."""
+        if self._kept is None:
+            tables = make()
+            if not torch.cuda.is_current_stream_capturing():
+                ready = torch.cuda.Event()
+                ready.record()
+                self._kept = (tables, ready, {stream()})
+            return tables
+        tables, ready, joined = self._kept
+        s = stream()
+        if s not in joined and not torch.cuda.is_current_stream_capturing():
+            current = torch.cuda.current_stream()
+            current.wait_event(ready)
+            _mark_used(tables, current)
+            joined.add(s)
+        return tables
+
+
+def _mark_used(tables, on):
+    if isinstance(tables, tuple):
+        for t in tables:
+            _mark_used(t, on)
+    elif tables is not None:
+        tables.record_stream(on)
+
+
 def reduction_buffer(device):
     """Memory of one two-pass reduction: its result, then fs_reduce_partials()
     doubles.  Allocated per call, so that reductions on several streams or

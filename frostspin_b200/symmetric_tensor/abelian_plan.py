@@ -26,6 +26,7 @@ relies on for Z2 = {-128, 0} (examples/ising_classical_ctmrg.py:369-378).
 
 import numpy as np
 
+from .. import device as dev
 from .._native import FS_PERM_MAXR, PERM_EB_DTYPE, PERM_TASK_DTYPE
 
 TASK_CHUNK = 8192
@@ -317,7 +318,7 @@ def build_abelian_permute_plan(
     plan.tasks = _make_tasks(ebs)
     plan.tiles = _make_tile_tasks(ebs)
     plan.in_len = int(in_len)
-    plan.device_tables = None
+    plan.device_tables = dev.KeptTables()
     return plan
 
 

@@ -187,8 +187,7 @@ class AbelianSymmetricTensor(SymmetricTensor):
         if plan.size and linalg.defer_permute(tables, self._data, out, 16.0 * plan.size):
             return out, plan.offsets, plan.block_shapes, plan.block_irreps
         if plan.size:
-            if plan.device_tables is None:
-                plan.device_tables = linalg.upload_copies(tables)
+            d_tables = plan.device_tables.get(lambda: linalg.upload_copies(tables))
             with instrument.region("permute", bytes=16.0 * plan.size):
-                linalg.run_copies(tables, plan.device_tables, self._data, out)
+                linalg.run_copies(tables, d_tables, self._data, out)
         return out, plan.offsets, plan.block_shapes, plan.block_irreps

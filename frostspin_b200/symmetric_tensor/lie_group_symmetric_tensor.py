@@ -162,15 +162,16 @@ class LieMap:
         "out_irreps", "in_len", "fused", "fused_coeffs",
     )
 
+    def _upload(self):
+        fz = self.fused
+        return (
+            linalg.upload_copies(self.gather), linalg.upload_copies(self.scatter),
+            dev.upload_f64(self.u_host),
+            None if fz is None else tuple(dev.upload(a) for a in fz),
+        )
+
     def run(self, src, out=None):
-        if self.device is None:
-            fz = self.fused
-            self.device = (
-                linalg.upload_copies(self.gather), linalg.upload_copies(self.scatter),
-                dev.upload_f64(self.u_host),
-                None if fz is None else tuple(dev.upload(a) for a in fz),
-            )
-        d_gather, d_scatter, d_u, d_fz = self.device
+        d_gather, d_scatter, d_u, d_fz = self.device.get(self._upload)
         if out is None:
             out = dev.zeros_f64(self.out_size) if self.zero_out else dev.empty_f64(self.out_size)
         if src.numel() < self.in_len:
@@ -653,7 +654,7 @@ class LieGroupSymmetricTensor(NonAbelianSymmetricTensor):
         m.M, m.N, m.K = st["M"][rest], E[rest], st["K"][rest]
         m.u_off, m.x_off, m.u_host = st["u_off"][rest], x_off[rest], st["u_host"]
         m.fused, m.fused_coeffs = fused, fused_coeffs
-        m.device = None
+        m.device = dev.KeptTables()
         m.out_offsets, m.out_shapes, m.out_irreps = out_offsets, out_shapes, st["bi_out"]
         m.in_len = int(self._data.numel())
         _MAP_CACHE[key] = m
@@ -857,7 +858,7 @@ class LieGroupSymmetricTensor(NonAbelianSymmetricTensor):
         m.x_size, m.out_size = x_size, out_size
         m.M, m.N, m.K = st["M"], E, st["K"]
         m.u_off, m.x_off, m.u_host = st["u_off"], x_off, st["u_host"]
-        m.device = None
+        m.device = dev.KeptTables()
         return m
 
     def _to_dense_map(self):

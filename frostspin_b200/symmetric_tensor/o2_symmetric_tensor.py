@@ -187,7 +187,7 @@ class _Recombine:
         self.offsets = []
         self.shapes = []
         self.irreps = []
-        self.device_tables = None
+        self.device_tables = dev.KeptTables()
         self._all_terms = []
 
     def _push(self, arr, kind):
@@ -272,10 +272,8 @@ class _Recombine:
         out = dev.empty_f64(self.out_len)
         if self.blocks.size == 0 or self.out_len == 0:
             return out
-        if self.device_tables is None:
-            self.device_tables = (dev.upload(self.blocks), dev.upload(self.index),
-                                  dev.upload(self.coef))
-        d_blocks, d_index, d_coef = self.device_tables
+        d_blocks, d_index, d_coef = self.device_tables.get(
+            lambda: (dev.upload(self.blocks), dev.upload(self.index), dev.upload(self.coef)))
         with instrument.region("o2_recombine", bytes=16.0 * self.out_len):
             for start in range(0, self.blocks.size, _MAX_BLOCKS_PER_CALL):
                 cnt = min(_MAX_BLOCKS_PER_CALL, self.blocks.size - start)
