@@ -19,8 +19,8 @@ std::atomic<long long> g_spin_limit{kDefaultSpinLimit};
 
 struct SmemConfig {
     std::mutex mutex;
-    // (kernel, device) pairs already configured, with the bytes set
-    static constexpr int kSlots = 64;
+    // one entry per (kernel, device) configured, with the largest bytes set
+    static constexpr int kSlots = 256;
     const void* func[kSlots] = {};
     int device[kSlots] = {};
     int bytes[kSlots] = {};
@@ -48,22 +48,34 @@ int num_sms() {
     return n;
 }
 
+// The limit of a kernel only ever rises: another thread may be between its own
+// call and its launch with more bytes.
 int configure_smem(const void* func, int bytes) {
     const int d = current_device();
     std::lock_guard<std::mutex> lock(g_smem.mutex);
-    for (int i = 0; i < g_smem.used; ++i)
-        if (g_smem.func[i] == func && g_smem.device[i] == d && g_smem.bytes[i] >= bytes)
-            return FS_OK;
-    cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    int at = 0;
+    while (at < g_smem.used && !(g_smem.func[at] == func && g_smem.device[at] == d)) ++at;
+    cudaError_t e = cudaSuccess;
+    int now = 0;   // bytes set so far
+    if (at < g_smem.used) {
+        now = g_smem.bytes[at];
+    } else if (at == SmemConfig::kSlots) {
+        cudaFuncAttributes attr;
+        e = cudaFuncGetAttributes(&attr, func);
+        if (e == cudaSuccess) now = attr.maxDynamicSharedSizeBytes;
+    }
+    if (e == cudaSuccess && now >= bytes) return FS_OK;
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) {
         set_last_cuda_error(e);
         return FS_ERR_CUDA;
     }
-    if (g_smem.used < SmemConfig::kSlots) {
-        g_smem.func[g_smem.used] = func;
-        g_smem.device[g_smem.used] = d;
-        g_smem.bytes[g_smem.used] = bytes;
-        ++g_smem.used;
+    if (at < SmemConfig::kSlots) {
+        g_smem.func[at] = func;
+        g_smem.device[at] = d;
+        g_smem.bytes[at] = bytes;
+        if (at == g_smem.used) ++g_smem.used;
     }
     return FS_OK;
 }

@@ -707,7 +707,10 @@ extern "C" int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_
     }
     const int bytes = static_cast<int>(sizeof(double)) *
                       (list.a_doubles + fsb::kWideWarps * fsb::kWideBufC);
-    const int st = fsb::configure_smem(reinterpret_cast<const void*>(fsb::k_dgemm_wide), bytes);
+    // one limit for every size: one CTA runs per SM whatever it asks for
+    const int st = fsb::configure_smem(reinterpret_cast<const void*>(fsb::k_dgemm_wide),
+                                       static_cast<int>(sizeof(double)) *
+                                           (fsb::kWideMaxA + fsb::kWideWarps * fsb::kWideBufC));
     if (st != FS_OK) return st;
     fsb::k_dgemm_wide<<<fsb::num_sms(), fsb::kWideThreads, bytes, fsb::as_stream(stream)>>>(list);
     return fsb::launch_status();
