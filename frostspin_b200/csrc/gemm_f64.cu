@@ -452,7 +452,9 @@ extern "C" int fs_grouped_dgemm_uniform(const FsGemmProblem* d_problems, int64_t
 // there (L2 write sectors 4 times the ideal), 201 us here.
 //
 // CTA b takes an equal share of the estimated time of all strips, problem by
-// problem, so it loads one or two A.
+// problem, so it loads one or two A.  The host adds up the times: with every CTA
+// counting the strips of every problem, 30 sectors of 8 x 8 on 0.1 M columns took
+// 42 us, 17 us now.
 namespace fsb {
 
 constexpr int kWideWarps = 16;
@@ -464,6 +466,7 @@ constexpr int kWideMaxA = 227 * 1024 / 8 - kWideWarps * kWideBufC;
 
 struct WideList {
     FsGemmProblem v[kWideMaxProblems];
+    int64_t pos[kWideMaxProblems + 1];   // time of all strips before each problem
     int32_t n_problems;
     int32_t a_doubles;   // shared doubles of the largest op(A)
 };
@@ -487,12 +490,20 @@ __host__ __device__ __forceinline__ int wide_ld(int K) {
 __host__ __device__ __forceinline__ int wide_cols(int K) {
     return wide_steps(K) <= 4 ? 32 : wide_steps(K) <= 16 ? 16 : 8;
 }
-// relative time of a strip: FP64 FMAs at 64 per cycle and SM, bytes at 23; the
-// shorter of the two is about half hidden
+__host__ __device__ __forceinline__ int64_t wide_strip_count(int N, int K) {
+    return (static_cast<int64_t>(N) + wide_cols(K) - 1) / wide_cols(K);
+}
+// relative time of a strip, in 1 / 2944 cycles of an SM: FP64 FMAs at 64 per cycle,
+// bytes at 23, the shorter of the two about half hidden, and what a strip takes
+// whatever its size (64 cycles; 0 and 16 left the CTAs of the smallest sectors
+// late: 40 ragged sectors of M <= 150 on 0.3 M columns 9 % and 6 % slower).
+// Rounded to whole cycles of a column, a strip of 1 x 1 had counted 1 / 129 of one
+// of 4 x 3: 9 sectors of up to 4 x 3 on 0.3 M columns 93 us, 15 us now.
+constexpr int64_t kWideStrip = 2944 * 64;
 __host__ __device__ __forceinline__ int64_t wide_cost(int M, int K) {
-    const int64_t math = static_cast<int64_t>(wide_rows(M)) * wide_k(K) / 64;
-    const int64_t mem = static_cast<int64_t>(M + K) * 8 / 23;
-    return (math > mem ? 2 * math + mem : 2 * mem + math) * wide_cols(K) + 1;
+    const int64_t math = static_cast<int64_t>(wide_rows(M)) * wide_k(K) * 23;
+    const int64_t mem = (static_cast<int64_t>(M) + K) * 8 * 64;
+    return (math > mem ? 2 * math + mem : 2 * mem + math) * wide_cols(K) + kWideStrip;
 }
 
 // The columns n0 .. n0 + 8 NT - 1 of op(B) as DMMA fragments, one k step at a
@@ -619,26 +630,18 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     double* sa = wide_smem;
     double* sc = wide_smem + list.a_doubles + threadIdx.x / 32 * kWideBufC;
 
-    int64_t total = 0;
-    for (int i = 0; i < list.n_problems; ++i) {
-        const FsGemmProblem& p = list.v[i];
-        const int cols = wide_cols(p.K);
-        total += (static_cast<int64_t>(p.N) + cols - 1) / cols * wide_cost(p.M, p.K);
-    }
+    const int64_t total = list.pos[list.n_problems];
     const int64_t lo = total / gridDim.x * blockIdx.x +
                        total % gridDim.x * blockIdx.x / gridDim.x;
     const int64_t hi = total / gridDim.x * (blockIdx.x + 1) +
                        total % gridDim.x * (blockIdx.x + 1) / gridDim.x;
-    int64_t pos = 0;
 #pragma unroll 1
-    for (int i = 0; i < list.n_problems && pos < hi; ++i) {
+    for (int i = 0; i < list.n_problems && list.pos[i] < hi; ++i) {
+        if (list.pos[i + 1] <= lo) continue;   // its divisions would cost as much as a strip
         const FsGemmProblem& p = list.v[i];
-        const int64_t cost = wide_cost(p.M, p.K);
-        const int cols = wide_cols(p.K);
-        const int64_t strips = (static_cast<int64_t>(p.N) + cols - 1) / cols;
+        const int64_t cost = wide_cost(p.M, p.K), pos = list.pos[i];
         const int64_t first = lo > pos ? (lo - pos + cost - 1) / cost : 0;
-        const int64_t last = min((hi - pos + cost - 1) / cost, strips);
-        pos += strips * cost;
+        const int64_t last = min((hi - pos + cost - 1) / cost, wide_strip_count(p.N, p.K));
         if (first >= last || p.M <= 0) continue;
         const int m8 = wide_rows(p.M), k4 = wide_k(p.K), ld = wide_ld(p.K);
         __syncthreads();   // the previous problem's A has been read
@@ -697,6 +700,7 @@ extern "C" int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_
     memcpy(list.v, h_problems, sizeof(FsGemmProblem) * static_cast<size_t>(n_problems));
     list.n_problems = static_cast<int32_t>(n_problems);
     list.a_doubles = 0;
+    list.pos[0] = 0;
     for (int64_t i = 0; i < n_problems; ++i) {
         const FsGemmProblem& p = h_problems[i];
         if (p.M < 0 || p.N < 0 || p.K < 0) return FS_ERR_INVALID_ARG;
@@ -704,6 +708,7 @@ extern "C" int fs_grouped_dgemm_wide(const FsGemmProblem* h_problems, int64_t n_
         const int64_t a = static_cast<int64_t>(fsb::wide_rows(p.M)) * fsb::wide_ld(p.K);
         if (a > fsb::kWideMaxA) return FS_ERR_TOO_LARGE;
         if (a > list.a_doubles) list.a_doubles = static_cast<int32_t>(a);
+        list.pos[i + 1] = list.pos[i] + fsb::wide_strip_count(p.N, p.K) * fsb::wide_cost(p.M, p.K);
     }
     const int bytes = static_cast<int>(sizeof(double)) *
                       (list.a_doubles + fsb::kWideWarps * fsb::kWideBufC);
