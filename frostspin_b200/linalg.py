@@ -503,24 +503,42 @@ _STREAM_MAX_K = 256   # longest K of a launch that goes to the streaming kernel
 
 
 _WIDE = {}
-# Two strips of 16 columns for every warp.  Streaming against wide kernel, N =
-# 40 000 and 80 000: M = K = 50 20.0 / 21.4 and 35.4 / 31.3 us, 150 x 40 42 / 34
-# and 82 / 57 us, 60 x 120 68 / 70 us at 80 000.
-_WIDE_COLUMNS = 148 * 16 * 16 * 2
+_WIDE_COLUMNS = 148 * 16 * 16   # a strip of 16 columns for every warp of the wide kernel
+# Strips a warp from which the wide kernel pays: 2 up to 3 problems, 3 beyond (more
+# A to load for each CTA); 4/3 as many from K = 41 on, where the streaming kernel
+# has hidden its pipeline fill, and 7/3 as many from K = 17 on when the rows fill
+# its 64 x 64 tiles.  Time of the streaming kernel over the wide one's, lowest and
+# geometric mean over 1, 3, 9, 18 and 40 even and ragged sectors of M = 4 to 150, K =
+# 3 to 104: 76 000 columns 0.72 and 1.09 (up to 3 sectors 0.82 and 1.18); 120 000
+# 0.79 and 1.22 (K <= 40, rows not filled, 0.97 and 1.28); 160 000 0.90 and 1.30;
+# 300 000 1.07 and 1.49.  Rows that fill their tiles, K > 16: 120 000 0.79 and 0.95,
+# 200 000 0.92 and 1.06, 300 000 1.08 and 1.18.
+_WIDE_STRIPS, _WIDE_STRIPS_FEW, _WIDE_FEW = 3, 2, 3
+_WIDE_LONG_K = 41
+_WIDE_FILL, _WIDE_FILL_K = 0.87, 17
 
 
 def _wide(arr):
     """Whether a launch goes to the wide kernel: op(A) of every problem in shared
     memory, and columns enough for all its warps."""
+    columns = int(arr["N"].sum())
+    need = _WIDE_COLUMNS * (_WIDE_STRIPS_FEW if arr.size <= _WIDE_FEW else _WIDE_STRIPS)
+    if columns < need:
+        return False
     if not _WIDE:
         _WIDE["limits"] = _native.dgemm_wide_limits()
     max_n, max_k, max_a = _WIDE["limits"]
-    if arr.size > max_n or int(arr["K"].max()) > max_k:
+    k = int(arr["K"].max())
+    if arr.size > max_n or k > max_k:
         return False
-    if int(arr["N"].sum()) < _WIDE_COLUMNS:
+    if k >= _WIDE_LONG_K and 3 * columns < 4 * need:
+        return False
+    M, N = arr["M"].astype(np.int64), arr["N"].astype(np.int64)
+    if k >= _WIDE_FILL_K and 3 * columns < 7 * need and (
+            (_pad(M, 8) * N).sum() > _WIDE_FILL * (_pad(M, 64) * N).sum()):
         return False
     # rows in eights, k steps of 4 in pairs, and 4 doubles against bank conflicts
-    a = _pad(arr["M"].astype(np.int64), 8) * (_pad(arr["K"].astype(np.int64), 8) + 4)
+    a = _pad(M, 8) * (_pad(arr["K"].astype(np.int64), 8) + 4)
     return int(a.max()) <= max_a
 
 
@@ -550,7 +568,7 @@ def _launch_dgemm(arr):
     FS_DGEMM_LIST_MAX problems travel with the launch; longer tables, and
     launches of the per-tile kernel from _TABLE_FLOPS on, go through device memory
     with their tile list."""
-    if int(arr["N"].sum()) >= _WIDE_COLUMNS and _wide(arr):
+    if _wide(arr):
         arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
         _native.call("fs_grouped_dgemm_wide", arr.ctypes.data, arr.size, dev.stream())
         return
