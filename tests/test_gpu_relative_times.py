@@ -28,6 +28,18 @@ def _best_us(*calls, reps=7):
     return best
 
 
+@pytest.mark.parametrize("shape", [(1, 4_000_000), (4_000_000, 1), (3, 1_000_001), (900_001, 7)])
+def test_thin_crossed_contraction(shape):
+    """A thin block against one of the other storage order: within twice the time
+    of the same block against one of its own (6 times with 64 x 64 tiles)."""
+    m, n = shape
+    x, y = (torch.randn(m * n, dtype=torch.float64, device="cuda") for _ in range(2))
+    same, crossed = _best_us(
+        lambda: linalg.pair_contract(x, y, [(0, 0, m, n, False, True, 1.0)]),
+        lambda: linalg.pair_contract(x, y, [(0, 0, m, n, False, False, 1.0)]))
+    assert crossed <= 2 * same, (crossed, same)
+
+
 def _sectors(shapes):
     arr = np.zeros(len(shapes), dtype=_native.GEMM_PROBLEM_DTYPE)
     keep = []
