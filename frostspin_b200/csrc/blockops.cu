@@ -186,7 +186,11 @@ constexpr int kRowStep = kOpThreads / 32;        // tile rows a pass covers
 // Contractions of 9 M coefficients, tiles against this: side 1 664-724 / 42 us, 4
 // 181-198 / 43 us, 8 101-108 / 44 us, 16 65 / 46 us; of 0.3 M: 8 15.3 / 13.3 us, 12
 // 15.4 / 15.3 us, 16 13.3 / 15.3 us.
+// Diagonal products of 9 M coefficients: side 1 745-845 / 34-44 us, 4 198-222 / 34-38
+// us, 8 103-120 / 37 us, 16 56-69 / 38-69 us (the output in interleaved runs); of
+// 0.3 M: 8 11.1 / 11.2 us, 10 10.2-11.2 / 11.2-13.2 us.
 constexpr int kThin = 16;
+constexpr int kThinDiag = 10;
 
 // Element f of a buffer with rows of `width` is element (f % width) * length + f / width
 // of the buffer of the other order.  Rows of a run of kUnit elements come from
@@ -316,9 +320,13 @@ __global__ void __launch_bounds__(kOpThreads, 2)
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
+__device__ __forceinline__ bool diag_tiled(const FsDiagBlock& d) {
+    return d.x_trans && d.m >= kThinDiag && d.n >= kThinDiag;
+}
+
 __device__ __forceinline__ int64_t diag_units(const FsDiagBlock& d) {
     const int64_t m = d.m, n = d.n;
-    return d.x_trans ? ceil_div(m, kTile) * ceil_div(n, kTile) : ceil_div(m * n, kUnit);
+    return diag_tiled(d) ? ceil_div(m, kTile) * ceil_div(n, kTile) : ceil_div(m * n, kUnit);
 }
 
 // Bound by HBM (16 bytes per coefficient).  The row of an element comes from
@@ -381,6 +389,39 @@ __global__ void __launch_bounds__(kOpThreads, 4)
                         const int t = (h + k) * kOpThreads + threadIdx.x;
                         if (t < cnt) po[f0 + t] = v[k] * w[k];
                     }
+                }
+            }
+        } else if (!diag_tiled(db)) {
+            // x has n rows of m, the output m rows of n
+            const bool by_out = n <= m;   // the output's rows are the short ones
+            const Turned t = turned(by_out ? n : m, by_out ? m : n);
+            const bool major = by_out == (db.left != 0);   // the weight goes with f / width
+            for (int64_t u = lo; u < hi; ++u) {
+                const int64_t f0 = u * kUnit, i0 = f0 / t.width;
+                const uint32_t j0 = static_cast<uint32_t>(f0 - i0 * t.width);
+                const int64_t left = m * n - f0;
+                const int cnt = left < kUnit ? static_cast<int>(left) : kUnit;
+#pragma unroll
+                for (int h = 0; h < kPerThread; h += kBatch) {
+                    double v[kBatch], w[kBatch];
+                    int64_t at[kBatch];
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) {
+                        const int e = (h + k) * kOpThreads + threadIdx.x;
+                        v[k] = w[k] = 0.0;
+                        if (e < cnt) {
+                            const uint32_t l = j0 + e, r = fast_div(l, t.mul, t.shift);
+                            const uint32_t c = l - r * t.width;
+                            const int64_t turn = c * t.length + i0 + r;
+                            v[k] = __ldg(px + (by_out ? turn : f0 + e));
+                            w[k] = __ldg(pd + (major ? i0 + r : static_cast<int64_t>(c)));
+                            at[k] = by_out ? f0 + e : turn;
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k)
+                        if ((h + k) * kOpThreads + static_cast<int>(threadIdx.x) < cnt)
+                            po[at[k]] = v[k] * w[k];
                 }
             }
         } else {

@@ -40,6 +40,20 @@ def test_thin_crossed_contraction(shape):
     assert crossed <= 2 * same, (crossed, same)
 
 
+@pytest.mark.parametrize("left", [False, True])
+@pytest.mark.parametrize("shape", [(1, 4_000_000), (4_000_000, 1), (3, 1_000_001), (900_001, 4)])
+def test_thin_transposed_diagonal_product(shape, left):
+    """The same for the product of a transposed block with a diagonal (up to 15
+    times with 64 x 64 tiles)."""
+    m, n = shape
+    x = torch.randn(m * n, dtype=torch.float64, device="cuda")
+    d = torch.randn(max(m, n), dtype=torch.float64, device="cuda")
+    same, turned = _best_us(
+        lambda: linalg.diag_mul(x, d, [(0, 0, 0, m, n, False, left)], m * n),
+        lambda: linalg.diag_mul(x, d, [(0, 0, 0, m, n, True, left)], m * n))
+    assert turned <= 2 * same, (turned, same)
+
+
 def _sectors(shapes):
     arr = np.zeros(len(shapes), dtype=_native.GEMM_PROBLEM_DTYPE)
     keep = []

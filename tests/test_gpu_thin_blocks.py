@@ -1,5 +1,6 @@
 """Thin blocks whose two sides run in different storage orders, at the edges of
-the element-wise form: sides around its limit of 16, runs of 4096 elements that
+the element-wise forms: sides around their limits of 16 (contractions) and 10
+(diagonal products), runs of 4096 elements that
 end inside a row, odd offsets, infinities beside the block.  A product is one
 rounding; a sum of n terms differs from numpy's by at most n eps sum |terms|."""
 
@@ -10,7 +11,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1), (1, 4096), (4097, 1), (2, 2048), (2, 2049), (3, 1365), (1366, 3), (5, 9000),
-          (7, 12293), (12293, 7), (15, 3000), (3001, 15), (16, 300), (300, 16), (15, 15), (2, 1)]
+          (7, 12293), (12293, 7), (15, 3000), (3001, 15), (16, 300), (300, 16), (15, 15), (2, 1),
+          (9, 5000), (4999, 9), (10, 500), (500, 10)]
 EPS = np.finfo(np.float64).eps
 
 
@@ -44,3 +46,25 @@ def test_crossed_contraction(trans, gap):
     terms = np.concatenate(terms)
     got = float(linalg.pair_contract(da, db, pairs))
     assert abs(got - terms.sum()) <= terms.size * EPS * np.abs(terms).sum()
+
+
+@pytest.mark.parametrize("left", [False, True])
+@pytest.mark.parametrize("gap", [1, 2])
+def test_diagonal_product_of_transposed_blocks(left, gap):
+    from frostspin_b200 import linalg
+
+    rng = np.random.default_rng(gap)
+    host, dx, off = _buffer(rng, gap)
+    want = np.full(host.size, np.nan)
+    entries, diag, at = [], [], 0
+    for o, (m, n) in zip(off, SHAPES, strict=True):
+        d = rng.standard_normal(m if left else n)
+        x = host[o:o + m * n].reshape(n, m).T
+        want[o:o + m * n] = (d[:, None] * x if left else x * d).ravel()
+        entries.append((o, o, at, m, n, True, left))
+        diag.append(d)
+        at += d.size
+    dd = torch.from_numpy(np.concatenate(diag)).cuda()
+    got = linalg.diag_mul(dx, dd, entries, host.size).cpu().numpy()
+    inside = ~np.isnan(want)
+    assert np.array_equal(got[inside], want[inside])
