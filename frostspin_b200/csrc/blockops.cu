@@ -180,17 +180,20 @@ constexpr int kUnit = kTile * kTile;
 constexpr int kPerThread = kUnit / kOpThreads;   // 16
 constexpr int kRowStep = kOpThreads / 32;        // tile rows a pass covers
 
-// Blocks whose two sides run in different orders and whose shorter side is below
-// kThin leave most of a tile empty: they go element by element along the buffer
-// whose rows are short (Turned), the other buffer in a few interleaved runs.
+// Long blocks whose two sides run in different orders and whose shorter side is
+// below kThin leave most of their tiles empty: they go element by element along the
+// buffer whose rows are short (Turned), the other buffer in a few interleaved runs.
 // Contractions of 9 M coefficients, tiles against this: side 1 664-724 / 42 us, 4
 // 181-198 / 43 us, 8 101-108 / 44 us, 16 65 / 46 us; of 0.3 M: 8 15.3 / 13.3 us, 12
-// 15.4 / 15.3 us, 16 13.3 / 15.3 us.
-// Diagonal products of 9 M coefficients: side 1 745-845 / 34-44 us, 4 198-222 / 34-38
-// us, 8 103-120 / 37 us, 16 56-69 / 38-69 us (the output in interleaved runs); of
-// 0.3 M: 8 11.1 / 11.2 us, 10 10.2-11.2 / 11.2-13.2 us.
+// 15.4 / 15.3 us, 16 13.3 / 15.3 us.  Diagonal products of 9 M: side 1 745-845 / 36-46
+// us, 4 198-222 / 36-38 us, 8 103-120 / 36-38 us; of 0.3 M: 8 11.1 / 11.2 us.
 constexpr int kThin = 16;
 constexpr int kThinDiag = 10;
+
+// A side of up to kUnit wastes no more than kTile tiles, less than a launch.
+__device__ __host__ __forceinline__ bool is_thin(int64_t m, int64_t n, int limit) {
+    return (m < limit || n < limit) && (m > kUnit || n > kUnit);
+}
 
 // Element f of a buffer with rows of `width` is element (f % width) * length + f / width
 // of the buffer of the other order.  Rows of a run of kUnit elements come from
@@ -210,7 +213,7 @@ __device__ __forceinline__ Turned turned(int64_t width, int64_t length) {
 __device__ __forceinline__ int pair_kind(const FsPairBlock& p) {
     if (p.b_off < 0) return 0;
     if ((p.a_trans != 0) != (p.b_trans != 0)) return 1;
-    return p.m < kThin || p.n < kThin ? 3 : 2;
+    return is_thin(p.m, p.n, kThin) ? 3 : 2;
 }
 
 __device__ __forceinline__ int64_t pair_units(const FsPairBlock& p) {
@@ -320,13 +323,19 @@ __global__ void __launch_bounds__(kOpThreads, 2)
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
-__device__ __forceinline__ bool diag_tiled(const FsDiagBlock& d) {
-    return d.x_trans && d.m >= kThinDiag && d.n >= kThinDiag;
+__host__ __device__ __forceinline__ bool diag_thin(const FsDiagBlock& d) {
+    return d.x_trans && is_thin(d.m, d.n, kThinDiag);
 }
 
+// units of a block in k_diag_mul, and in k_diag_thin
 __device__ __forceinline__ int64_t diag_units(const FsDiagBlock& d) {
     const int64_t m = d.m, n = d.n;
-    return diag_tiled(d) ? ceil_div(m, kTile) * ceil_div(n, kTile) : ceil_div(m * n, kUnit);
+    if (diag_thin(d)) return 0;
+    return d.x_trans ? ceil_div(m, kTile) * ceil_div(n, kTile) : ceil_div(m * n, kUnit);
+}
+
+__device__ __forceinline__ int64_t diag_thin_units(const FsDiagBlock& d) {
+    return diag_thin(d) ? ceil_div(static_cast<int64_t>(d.m) * d.n, kUnit) : 0;
 }
 
 // Bound by HBM (16 bytes per coefficient).  The row of an element comes from
@@ -391,39 +400,6 @@ __global__ void __launch_bounds__(kOpThreads, 4)
                     }
                 }
             }
-        } else if (!diag_tiled(db)) {
-            // x has n rows of m, the output m rows of n
-            const bool by_out = n <= m;   // the output's rows are the short ones
-            const Turned t = turned(by_out ? n : m, by_out ? m : n);
-            const bool major = by_out == (db.left != 0);   // the weight goes with f / width
-            for (int64_t u = lo; u < hi; ++u) {
-                const int64_t f0 = u * kUnit, i0 = f0 / t.width;
-                const uint32_t j0 = static_cast<uint32_t>(f0 - i0 * t.width);
-                const int64_t left = m * n - f0;
-                const int cnt = left < kUnit ? static_cast<int>(left) : kUnit;
-#pragma unroll
-                for (int h = 0; h < kPerThread; h += kBatch) {
-                    double v[kBatch], w[kBatch];
-                    int64_t at[kBatch];
-#pragma unroll
-                    for (int k = 0; k < kBatch; ++k) {
-                        const int e = (h + k) * kOpThreads + threadIdx.x;
-                        v[k] = w[k] = 0.0;
-                        if (e < cnt) {
-                            const uint32_t l = j0 + e, r = fast_div(l, t.mul, t.shift);
-                            const uint32_t c = l - r * t.width;
-                            const int64_t turn = c * t.length + i0 + r;
-                            v[k] = __ldg(px + (by_out ? turn : f0 + e));
-                            w[k] = __ldg(pd + (major ? i0 + r : static_cast<int64_t>(c)));
-                            at[k] = by_out ? f0 + e : turn;
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < kBatch; ++k)
-                        if ((h + k) * kOpThreads + static_cast<int>(threadIdx.x) < cnt)
-                            po[at[k]] = v[k] * w[k];
-                }
-            }
         } else {
             const int64_t jt = ceil_div(n, kTile);
             for (int64_t u = lo; u < hi; ++u) {
@@ -449,6 +425,66 @@ __global__ void __launch_bounds__(kOpThreads, 4)
                         po[(i0 + i) * n + j0 + j] =
                             tile[j][i] * __ldg(pd + (db.left ? i0 + i : j0 + j));
                 }
+            }
+        }
+    }
+}
+
+// The thin transposed blocks of a list (x has n rows of m, the output m rows of n).
+// Apart, since this form took the registers that the others keep their loads in (9
+// blocks of 1200 x 1200 42 us, 46 us with all forms in one kernel).
+template <class Table>
+__global__ void __launch_bounds__(kOpThreads, 4)
+    k_diag_thin(const double* __restrict__ x, const double* __restrict__ diag,
+                double* __restrict__ out, const __grid_constant__ Table blocks,
+                int64_t n_blocks) {
+    int64_t mine = 0;
+    for (int64_t q = threadIdx.x; q < n_blocks; q += kOpThreads) mine += diag_thin_units(blocks[q]);
+    const int64_t total = block_total<kOpThreads>(mine);
+    const int64_t begin = total * blockIdx.x / gridDim.x;
+    const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
+    constexpr int kBatch = 8;
+    int64_t pos = 0;
+    for (int64_t q = 0; q < n_blocks && pos < end; ++q) {
+        const FsDiagBlock db = blocks[q];
+        const int64_t units = diag_thin_units(db);
+        const int64_t lo = begin > pos ? begin - pos : 0;
+        const int64_t hi = end - pos < units ? end - pos : units;
+        pos += units;
+        if (hi <= lo) continue;
+        const int64_t m = db.m, n = db.n;
+        const double* px = x + db.x_off;
+        const double* pd = diag + db.d_off;
+        double* po = out + db.out_off;
+        const bool by_out = n <= m;   // the output's rows are the short ones
+        const Turned t = turned(by_out ? n : m, by_out ? m : n);
+        const bool major = by_out == (db.left != 0);   // the weight goes with f / width
+        for (int64_t u = lo; u < hi; ++u) {
+            const int64_t f0 = u * kUnit, i0 = f0 / t.width;
+            const uint32_t j0 = static_cast<uint32_t>(f0 - i0 * t.width);
+            const int64_t left = m * n - f0;
+            const int cnt = left < kUnit ? static_cast<int>(left) : kUnit;
+#pragma unroll
+            for (int h = 0; h < kPerThread; h += kBatch) {
+                double v[kBatch], w[kBatch];
+                int64_t at[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    const int e = (h + k) * kOpThreads + threadIdx.x;
+                    v[k] = w[k] = 0.0;
+                    if (e < cnt) {
+                        const uint32_t l = j0 + e, r = fast_div(l, t.mul, t.shift);
+                        const uint32_t c = l - r * t.width;
+                        const int64_t turn = c * t.length + i0 + r;
+                        v[k] = __ldg(px + (by_out ? turn : f0 + e));
+                        w[k] = __ldg(pd + (major ? i0 + r : static_cast<int64_t>(c)));
+                        at[k] = by_out ? f0 + e : turn;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k)
+                    if ((h + k) * kOpThreads + static_cast<int>(threadIdx.x) < cnt)
+                        po[at[k]] = v[k] * w[k];
             }
         }
     }
@@ -536,13 +572,21 @@ int pair_contract(const double* d_a, const double* d_b, const Table& pairs, int6
     return fsb::launch_status();
 }
 
+// some, all: whether the list has thin blocks, and no others
 template <class Table>
 int diag_mul(const double* d_x, const double* d_diag, double* d_out, const Table& blocks,
-             int64_t n_blocks, void* stream) {
+             int64_t n_blocks, bool some, bool all, void* stream) {
     if (d_x == nullptr || d_diag == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
     // one wave of resident CTAs; CTAs without a unit return at once
-    fsb::k_diag_mul<<<4 * fsb::num_sms(), fsb::kOpThreads, 0, fsb::as_stream(stream)>>>(
-        d_x, d_diag, d_out, blocks, n_blocks);
+    const int grid = 4 * fsb::num_sms();
+    cudaStream_t s = fsb::as_stream(stream);
+    if (!all) {
+        fsb::k_diag_mul<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
+        const int st = fsb::launch_status();
+        if (st != FS_OK) return st;
+    }
+    if (!some) return FS_OK;
+    fsb::k_diag_thin<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
     return fsb::launch_status();
 }
 
@@ -610,14 +654,18 @@ extern "C" int fs_diag_mul(const double* d_x, const double* d_diag, double* d_ou
     if (n_blocks < 0) return FS_ERR_INVALID_ARG;
     if (n_blocks == 0) return FS_OK;
     if (d_blocks == nullptr) return FS_ERR_INVALID_ARG;
-    return diag_mul(d_x, d_diag, d_out, fsb::DeviceTable<FsDiagBlock>{d_blocks}, n_blocks, stream);
+    // the host cannot see the blocks: each kernel passes over the other's
+    return diag_mul(d_x, d_diag, d_out, fsb::DeviceTable<FsDiagBlock>{d_blocks}, n_blocks, true,
+                    false, stream);
 }
 
 extern "C" int fs_diag_mul_list(const double* d_x, const double* d_diag, double* d_out,
                                 const FsDiagBlock* h_blocks, int64_t n_blocks, void* stream) {
     const int st = list_status(h_blocks, n_blocks);
     if (st != FS_OK || n_blocks == 0) return st;
+    int64_t thin = 0;
+    for (int64_t i = 0; i < n_blocks; ++i) thin += fsb::diag_thin(h_blocks[i]);
     return diag_mul(d_x, d_diag, d_out,
                     fsb::inline_table<FsDiagBlock, FS_LIST_MAX>(h_blocks, n_blocks), n_blocks,
-                    stream);
+                    thin > 0, thin == n_blocks, stream);
 }

@@ -1,6 +1,6 @@
 """Thin blocks whose two sides run in different storage orders, at the edges of
-the element-wise forms: sides around their limits of 16 (contractions) and 10
-(diagonal products), runs of 4096 elements that
+the element-wise forms: short sides around their limits of 16 (contractions) and 10
+(diagonal products), long ones around 4096, runs of 4096 elements that
 end inside a row, odd offsets, infinities beside the block.  A product is one
 rounding; a sum of n terms differs from numpy's by at most n eps sum |terms|."""
 
@@ -10,9 +10,9 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(1, 1), (1, 4096), (4097, 1), (2, 2048), (2, 2049), (3, 1365), (1366, 3), (5, 9000),
-          (7, 12293), (12293, 7), (15, 3000), (3001, 15), (16, 300), (300, 16), (15, 15), (2, 1),
-          (9, 5000), (4999, 9), (10, 500), (500, 10)]
+SHAPES = [(1, 1), (1, 4096), (1, 4097), (4097, 1), (2, 4096), (2, 4097), (3, 4100), (4101, 3),
+          (5, 9000), (7, 12293), (12293, 7), (9, 5000), (4999, 9), (10, 4500), (4500, 10),
+          (15, 5001), (5000, 15), (16, 4097), (4097, 16), (15, 15), (2, 1), (3, 1365)]
 EPS = np.finfo(np.float64).eps
 
 
