@@ -90,6 +90,49 @@ __device__ __forceinline__ int64_t block_total(int64_t v) {
 
 __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// Where the share of a CTA that begins at unit `begin` of a list of n sizes starts:
+// an entry at or before it, and the units before that entry.  kScan: by a scan of
+// the list, for long ones: walking up to the share, a diagonal product of 96 blocks of
+// 40 x 40 took 31 us and one of 256 blocks of 20 x 20 74 us, 10 and 23 us now.  Short
+// lists are walked from their first entry (list_scanned).
+template <bool kScan, int T, class Size>
+__device__ __forceinline__ void list_start(int64_t n, int64_t begin, Size size, int64_t& first,
+                                           int64_t& pos) {
+    first = pos = 0;
+    if (!kScan) return;
+    __shared__ int64_t warp_sum[T / 32], found[2];
+    const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
+    if (threadIdx.x == 0) found[0] = n;
+    int64_t done = 0;
+    for (int64_t base = 0; base < n && done <= begin; base += T) {
+        const int64_t q = base + threadIdx.x;
+        const int64_t mine = q < n ? size(q) : 0;
+        int64_t upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o *= 2) {
+            const int64_t v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        __syncthreads();   // the sums of the previous entries have been read
+        if (lane == 31) warp_sum[wid] = upto;
+        __syncthreads();
+        upto += done;
+#pragma unroll
+        for (int w = 0; w < T / 32; ++w) {
+            if (w < wid) upto += warp_sum[w];
+            done += warp_sum[w];
+        }
+        if (upto - mine <= begin && begin < upto) {
+            found[0] = q;
+            found[1] = upto - mine;
+        }
+    }
+    __syncthreads();
+    // one value for the warp, so that the entries stay in uniform registers
+    first = __shfl_sync(0xffffffffu, found[0], 0);
+    pos = __shfl_sync(0xffffffffu, found[1], 0);
+}
+
 // mode 0: sum of squares, mode 1: plain sum.  Bound by HBM (8 bytes read per
 // coefficient).  The concatenated segments are cut into one contiguous share
 // per CTA, so that a CTA meets one or two segments whatever their number, and
@@ -101,7 +144,7 @@ __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 constexpr int kReduceThreads = 512;
 constexpr int kReduceUnroll = 8;
 
-template <int MODE, class Table>
+template <int MODE, bool kScan, class Table>
 __global__ void __launch_bounds__(kReduceThreads, 2)
     k_weighted_reduce(const double* __restrict__ x, const __grid_constant__ Table segs,
                       int64_t n_segs, double* __restrict__ partial) {
@@ -113,8 +156,10 @@ __global__ void __launch_bounds__(kReduceThreads, 2)
     const int64_t begin = share * blockIdx.x;
     const int64_t end = begin + share < total ? begin + share : total;
     double acc = 0.0;
-    int64_t pos = 0;
-    for (int64_t s = 0; s < n_segs && pos < end; ++s) {
+    int64_t s, pos;
+    list_start<kScan, kReduceThreads>(n_segs, begin,
+                                      [&](int64_t i) { return segs[i].length; }, s, pos);
+    for (; s < n_segs && pos < end; ++s) {
         const FsSegment sg = segs[s];
         const int64_t lo = begin > pos ? begin - pos : 0;
         const int64_t hi = end - pos < sg.length ? end - pos : sg.length;
@@ -231,7 +276,7 @@ __device__ __forceinline__ int64_t pair_units(const FsPairBlock& p) {
 // 64-bit divisions.  Here a thread issues its 32 loads of a tile pair before
 // the first use.  Two SU(2) corners of 13.1 M coefficients: 118 us before,
 // 37 us now.
-template <class Table>
+template <bool kScan, class Table>
 __global__ void __launch_bounds__(kOpThreads, 2)
     k_pair_contract(const double* __restrict__ a, const double* __restrict__ b,
                     const __grid_constant__ Table pairs, int64_t n_pairs,
@@ -244,8 +289,10 @@ __global__ void __launch_bounds__(kOpThreads, 2)
     const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
     const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
     double acc = 0.0;
-    int64_t pos = 0;
-    for (int64_t q = 0; q < n_pairs && pos < end; ++q) {
+    int64_t q, pos;
+    list_start<kScan, kOpThreads>(n_pairs, begin,
+                                  [&](int64_t i) { return pair_units(pairs[i]); }, q, pos);
+    for (; q < n_pairs && pos < end; ++q) {
         const FsPairBlock pb = pairs[q];
         const int64_t units = pair_units(pb);
         const int64_t lo = begin > pos ? begin - pos : 0;
@@ -344,7 +391,7 @@ __device__ __forceinline__ int64_t diag_thin_units(const FsDiagBlock& d) {
 // F-order inputs go through a shared tile.  12.2 M coefficients in 9 blocks:
 // 63 us before (a 64-bit division per element, one load at a time),
 // 36 us now.
-template <class Table>
+template <bool kScan, class Table>
 __global__ void __launch_bounds__(kOpThreads, 4)
     k_diag_mul(const double* __restrict__ x, const double* __restrict__ diag,
                double* __restrict__ out, const __grid_constant__ Table blocks,
@@ -357,8 +404,10 @@ __global__ void __launch_bounds__(kOpThreads, 4)
     const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
     const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
     constexpr int kBatch = 8;
-    int64_t pos = 0;
-    for (int64_t q = 0; q < n_blocks && pos < end; ++q) {
+    int64_t q, pos;
+    list_start<kScan, kOpThreads>(n_blocks, begin,
+                                  [&](int64_t i) { return diag_units(blocks[i]); }, q, pos);
+    for (; q < n_blocks && pos < end; ++q) {
         const FsDiagBlock db = blocks[q];
         const int64_t units = diag_units(db);
         const int64_t lo = begin > pos ? begin - pos : 0;
@@ -433,7 +482,7 @@ __global__ void __launch_bounds__(kOpThreads, 4)
 // The thin transposed blocks of a list (x has n rows of m, the output m rows of n).
 // Apart, since this form took the registers that the others keep their loads in (9
 // blocks of 1200 x 1200 42 us, 46 us with all forms in one kernel).
-template <class Table>
+template <bool kScan, class Table>
 __global__ void __launch_bounds__(kOpThreads, 4)
     k_diag_thin(const double* __restrict__ x, const double* __restrict__ diag,
                 double* __restrict__ out, const __grid_constant__ Table blocks,
@@ -444,8 +493,10 @@ __global__ void __launch_bounds__(kOpThreads, 4)
     const int64_t begin = total * blockIdx.x / gridDim.x;
     const int64_t end = total * (blockIdx.x + 1) / gridDim.x;
     constexpr int kBatch = 8;
-    int64_t pos = 0;
-    for (int64_t q = 0; q < n_blocks && pos < end; ++q) {
+    int64_t q, pos;
+    list_start<kScan, kOpThreads>(n_blocks, begin,
+                                  [&](int64_t i) { return diag_thin_units(blocks[i]); }, q, pos);
+    for (; q < n_blocks && pos < end; ++q) {
         const FsDiagBlock db = blocks[q];
         const int64_t units = diag_thin_units(db);
         const int64_t lo = begin > pos ? begin - pos : 0;
@@ -542,6 +593,23 @@ extern "C" int fs_pow(const double* d_x, double* d_y, int64_t n, double p, void*
 
 namespace {
 
+// Lists of more entries than these are scanned.  Walked against scanned: contraction
+// of 40 blocks of 40 x 40 16.6 / 11.6 us and of 4000 x 130 68.0 / 64.5 us, sum of
+// squares 16.5 / 9.8 and 35.4 / 35.0 us, diagonal product of 17 blocks of 40 x 40 8.4 /
+// 6.4 us, but of 9 of 1200 x 1200 37.5 / 39.1 us; 17 large blocks gain the sums nothing.
+constexpr int64_t kReduceWalk = 24, kPairWalk = 24, kDiagWalk = 12;
+
+// A table in device memory is longer, and scanned whatever its length.
+template <class Table>
+constexpr bool kInDevice = false;
+template <class T>
+constexpr bool kInDevice<fsb::DeviceTable<T>> = true;
+
+template <class Table>
+bool list_scanned(int64_t n, int64_t walk) {
+    return kInDevice<Table> || n > walk;
+}
+
 template <int MODE, class Table>
 int weighted_reduce(const double* d_x, const Table& segs, int64_t n_segs, double* d_partial,
                     int64_t n_partial, double* d_out, void* stream) {
@@ -549,8 +617,10 @@ int weighted_reduce(const double* d_x, const Table& segs, int64_t n_segs, double
     if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
     if (n_segs > 0 && d_x == nullptr) return FS_ERR_INVALID_ARG;
     cudaStream_t s = fsb::as_stream(stream);
-    fsb::k_weighted_reduce<MODE><<<fsb::kReducePartials, fsb::kReduceThreads, 0, s>>>(
-        d_x, segs, n_segs, d_partial);
+    const auto kernel = list_scanned<Table>(n_segs, kReduceWalk)
+                            ? fsb::k_weighted_reduce<MODE, true, Table>
+                            : fsb::k_weighted_reduce<MODE, kInDevice<Table>, Table>;
+    kernel<<<fsb::kReducePartials, fsb::kReduceThreads, 0, s>>>(d_x, segs, n_segs, d_partial);
     int st = fsb::launch_status();
     if (st != FS_OK) return st;
     fsb::k_final_sum<<<1, fsb::kOpThreads, 0, s>>>(d_partial, fsb::kReducePartials, d_out);
@@ -564,8 +634,10 @@ int pair_contract(const double* d_a, const double* d_b, const Table& pairs, int6
     if (d_partial == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
     if (n_pairs > 0 && d_a == nullptr) return FS_ERR_INVALID_ARG;
     cudaStream_t s = fsb::as_stream(stream);
-    fsb::k_pair_contract<<<fsb::kReducePartials, fsb::kOpThreads, 0, s>>>(d_a, d_b, pairs, n_pairs,
-                                                                          d_partial);
+    const auto kernel = list_scanned<Table>(n_pairs, kPairWalk)
+                            ? fsb::k_pair_contract<true, Table>
+                            : fsb::k_pair_contract<kInDevice<Table>, Table>;
+    kernel<<<fsb::kReducePartials, fsb::kOpThreads, 0, s>>>(d_a, d_b, pairs, n_pairs, d_partial);
     int st = fsb::launch_status();
     if (st != FS_OK) return st;
     fsb::k_final_sum<<<1, fsb::kOpThreads, 0, s>>>(d_partial, fsb::kReducePartials, d_out);
@@ -579,14 +651,19 @@ int diag_mul(const double* d_x, const double* d_diag, double* d_out, const Table
     if (d_x == nullptr || d_diag == nullptr || d_out == nullptr) return FS_ERR_INVALID_ARG;
     // one wave of resident CTAs; CTAs without a unit return at once
     const int grid = 4 * fsb::num_sms();
+    const bool scan = list_scanned<Table>(n_blocks, kDiagWalk);
     cudaStream_t s = fsb::as_stream(stream);
     if (!all) {
-        fsb::k_diag_mul<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
+        const auto kernel = scan ? fsb::k_diag_mul<true, Table>
+                                 : fsb::k_diag_mul<kInDevice<Table>, Table>;
+        kernel<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
         const int st = fsb::launch_status();
         if (st != FS_OK) return st;
     }
     if (!some) return FS_OK;
-    fsb::k_diag_thin<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
+    const auto kernel = scan ? fsb::k_diag_thin<true, Table>
+                             : fsb::k_diag_thin<kInDevice<Table>, Table>;
+    kernel<<<grid, fsb::kOpThreads, 0, s>>>(d_x, d_diag, d_out, blocks, n_blocks);
     return fsb::launch_status();
 }
 

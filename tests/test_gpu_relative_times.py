@@ -17,7 +17,8 @@ def _best_us(*calls, reps=7):
     best = [float("inf")] * len(calls)
     for r in range(reps + 1):
         for i, f in enumerate(calls):
-            flush.zero_()
+            for _ in range(8):      # long enough to hide the host's work of the call
+                flush.zero_()
             s, e = (torch.cuda.Event(enable_timing=True) for _ in range(2))
             s.record()
             f()
@@ -84,3 +85,24 @@ def test_wide_gemm_shares(shapes, monkeypatch):
     streaming, wide = _best_us(launch(1 << 60), launch(0))
     assert wide <= 0.8 * streaming, (wide, streaming)
     del keep
+
+
+@pytest.mark.parametrize("n", [96, 256])
+def test_many_blocks(n):
+    """A diagonal product and a contraction of many small blocks: within 4 times
+    the same over one block of their total size (walking up to a share took 6 to 9
+    times)."""
+    m = k = 40
+    x, y = (torch.randn(n * m * k, dtype=torch.float64, device="cuda") for _ in range(2))
+    d = torch.randn(n * m * k, dtype=torch.float64, device="cuda")
+    size = m * k
+    one, many = _best_us(
+        lambda: linalg.diag_mul(x, d, [(0, 0, 0, n * m, k, False, False)], x.numel()),
+        lambda: linalg.diag_mul(x, d, [(i * size, i * size, i * k, m, k, False, False)
+                                       for i in range(n)], x.numel()))
+    assert many <= 4 * one, (many, one)
+    one, many = _best_us(
+        lambda: linalg.pair_contract(x, y, [(0, 0, n * m, k, False, True, 1.0)]),
+        lambda: linalg.pair_contract(x, y, [(i * size, i * size, m, k, False, True, 1.0)
+                                            for i in range(n)]))
+    assert many <= 4 * one, (many, one)
