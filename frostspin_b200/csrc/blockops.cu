@@ -93,7 +93,7 @@ __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 // Where the share of a CTA that begins at unit `begin` of a list of n sizes starts:
 // an entry at or before it, and the units before that entry.  kScan: by a scan of
 // the list, for long ones: walking up to the share, a diagonal product of 96 blocks of
-// 40 x 40 took 31 us and one of 256 blocks of 20 x 20 74 us, 10 and 23 us now.  Short
+// 40 x 40 took 31 us and one of 256 blocks of 20 x 20 74 us, 10 and 27 us now.  Short
 // lists are walked from their first entry (list_scanned).
 template <bool kScan, int T, class Size>
 __device__ __forceinline__ void list_start(int64_t n, int64_t begin, Size size, int64_t& first,
@@ -135,8 +135,9 @@ __device__ __forceinline__ void list_start(int64_t n, int64_t begin, Size size, 
 
 // mode 0: sum of squares, mode 1: plain sum.  Bound by HBM (8 bytes read per
 // coefficient).  The concatenated segments are cut into one contiguous share
-// per CTA, so that a CTA meets one or two segments whatever their number, and
-// each thread keeps eight 16-byte loads in flight (64 KB per CTA, two CTAs per
+// per CTA, so that a CTA meets one or two segments whatever their number (200
+// segments of 1 to 4 elements 20 us; 97 us in shares of at least 512 elements, all in
+// one CTA), and each thread keeps eight 16-byte loads in flight (64 KB per CTA, two CTAs per
 // SM; the copy bandwidth needs about 40 KB per SM).  The share of CTA b is a
 // fixed function of the list, so the two-pass sum is deterministic.  12.2 M
 // coefficients in 9 segments: 76 us before (every CTA strode over every
@@ -151,8 +152,7 @@ __global__ void __launch_bounds__(kReduceThreads, 2)
     int64_t mine = 0;
     for (int64_t s = threadIdx.x; s < n_segs; s += kReduceThreads) mine += segs[s].length;
     const int64_t total = block_total<kReduceThreads>(mine);
-    int64_t share = ceil_div(total, gridDim.x);
-    if (share < kReduceThreads) share = kReduceThreads;
+    const int64_t share = ceil_div(total, gridDim.x);
     const int64_t begin = share * blockIdx.x;
     const int64_t end = begin + share < total ? begin + share : total;
     double acc = 0.0;

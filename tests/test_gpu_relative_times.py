@@ -106,3 +106,14 @@ def test_many_blocks(n):
         lambda: linalg.pair_contract(x, y, [(i * size, i * size, m, k, False, True, 1.0)
                                             for i in range(n)]))
     assert many <= 4 * one, (many, one)
+
+
+def test_sum_of_tiny_blocks():
+    """60 blocks of 2 elements: within twice the time of one block of 120 (3.5 times
+    while one CTA walked them all)."""
+    x = torch.randn(120, dtype=torch.float64, device="cuda")
+    one, many = _best_us(
+        lambda: [linalg.weighted_reduce(x, [0], [120], [1.0], squares=True) for _ in range(10)],
+        lambda: [linalg.weighted_reduce(x, 2 * np.arange(60), [2] * 60, [1.0] * 60, squares=True)
+                 for _ in range(10)])
+    assert many <= 2 * one, (many, one)
