@@ -18,6 +18,10 @@ constexpr int kPermThreads = 256;
 // coefficients in rows of ~40: 1253 us = 5.8 TB/s (1446 us with 4 loads, 1370
 // us with 8 loads and 3 CTAs, 1470 us with 16 loads and 2 CTAs).
 constexpr int kPermUnroll = 8;
+// Tasks of few entries, whose other loads would all be masked off: rank-6 tensors
+// of 0.14 and 0.75 M coefficients in small blocks 40.0 and 40.3 us (44.0 and 46.1
+// us with 8 loads, 38.0 and 40.1 us when every task had 4).
+constexpr int kPermUnrollShort = 2;
 constexpr int kPermMaxRows = 1024;   // rows per task (shared-memory row table)
 
 // One task = a range of rows of one elementary block, a row being one run along
@@ -33,6 +37,38 @@ constexpr int kPermMaxRows = 1024;   // rows per task (shared-memory row table)
 // kMulti: the EBs of several independent permutes in one launch; EB e reads
 // and writes the buffer pair bufs[e.pad] (the permutes of many CTMRG runs
 // advanced in lock step share one launch).
+//
+// perm_walk: phase 2 with U loads in flight.
+template <int U>
+__device__ __forceinline__ void perm_walk(const double* __restrict__ in, double* __restrict__ out,
+                                          const int64_t* row_src, const int64_t* row_dst,
+                                          uint32_t total, uint32_t L, uint32_t mL, uint32_t sL,
+                                          int64_t osL, int64_t nsL, bool zero_fill) {
+    for (uint32_t i0 = threadIdx.x; i0 < total; i0 += kPermThreads * U) {
+        double v[U];
+        int64_t dst[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t idx = i0 + u * kPermThreads;
+            dst[u] = -1;
+            v[u] = 0.0;
+            if (idx < total) {
+                const uint32_t row = fast_div(idx, mL, sL);
+                const uint32_t i = idx - row * L;
+                const int64_t rd = row_dst[row];
+                if (rd >= 0) {
+                    dst[u] = rd + static_cast<int64_t>(i) * nsL;
+                    if (!zero_fill) v[u] = __ldg(in + row_src[row] + static_cast<int64_t>(i) * osL);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (dst[u] >= 0) out[dst[u]] = v[u];
+        }
+    }
+}
+
 template <bool kMulti>
 __global__ void __launch_bounds__(kPermThreads, 4)
     k_perm_gather_t(const double* __restrict__ in0, int64_t in_len0, double* __restrict__ out0,
@@ -104,29 +140,11 @@ __global__ void __launch_bounds__(kPermThreads, 4)
         __syncthreads();
         const uint32_t total = static_cast<uint32_t>(nrows) * L;
         const uint32_t mL = e.divm[nd - 1], sL = e.divs[nd - 1];
-        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += kPermThreads * kPermUnroll) {
-            double v[kPermUnroll];
-            int64_t dst[kPermUnroll];
-#pragma unroll
-            for (int u = 0; u < kPermUnroll; ++u) {
-                const uint32_t idx = i0 + u * kPermThreads;
-                dst[u] = -1;
-                v[u] = 0.0;
-                if (idx < total) {
-                    const uint32_t row = fast_div(idx, mL, sL);
-                    const uint32_t i = idx - row * L;
-                    const int64_t rd = row_dst[row];
-                    if (rd >= 0) {
-                        dst[u] = rd + static_cast<int64_t>(i) * nsL;
-                        if (!zero_fill) v[u] = __ldg(in + row_src[row] + static_cast<int64_t>(i) * osL);
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kPermUnroll; ++u) {
-                if (dst[u] >= 0) out[dst[u]] = v[u];
-            }
-        }
+        if (total <= kPermUnrollShort * kPermThreads)
+            perm_walk<kPermUnrollShort>(in, out, row_src, row_dst, total, L, mL, sL, osL, nsL,
+                                        zero_fill);
+        else
+            perm_walk<kPermUnroll>(in, out, row_src, row_dst, total, L, mL, sL, osL, nsL, zero_fill);
     }
 }
 
