@@ -560,15 +560,16 @@ def _dgemm_list(name, arr, kind):
                  entry="fs_grouped_dgemm_list")
 
 
-def _launch_dgemm(arr):
-    """One DMMA launch over a problem table: the streaming kernel when every
+def _launch_dgemm(arr, wide=None):
+    """One DMMA launch over a problem table: the wide kernel where _wide says so
+    (wide: True or False to decide otherwise), the streaming kernel when every
     problem has the same transpose flags and a short K (pipeline fill and
     padded fragments dominate there), else the per-tile kernel (faster on long
     K, where it keeps a few registers more for the DMMA loop).  Up to
     FS_DGEMM_LIST_MAX problems travel with the launch; longer tables, and
     launches of the per-tile kernel from _TABLE_FLOPS on, go through device memory
     with their tile list."""
-    if _wide(arr):
+    if _wide(arr) if wide is None else wide:
         arr = arr[np.argsort(-arr["K"].astype(np.int64), kind="stable")]
         _native.call("fs_grouped_dgemm_wide", arr.ctypes.data, arr.size, dev.stream())
         return
@@ -592,13 +593,13 @@ def _launch_dgemm(arr):
                      n_tiles, dev.stream())
 
 
-def _dgemm(arr):
+def _dgemm(arr, wide=None):
     sk = _split_k(arr)
     if sk is None:
-        _launch_dgemm(arr)
+        _launch_dgemm(arr, wide)
         return
     arr, items, _work = sk   # the workspace lives until the reduction is queued
-    _launch_dgemm(arr)
+    _launch_dgemm(arr, wide)
     max_elems = int((items["M"].astype(np.int64) * items["N"]).max())
     if items.size <= _native.FS_SPLIT_LIST_MAX:
         _native.call("fs_splitk_reduce", items.ctypes.data, items.size, max_elems, dev.stream(),
