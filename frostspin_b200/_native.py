@@ -43,6 +43,7 @@ PERM_TASK_DTYPE = np.dtype(
 )
 
 FS_SU2_MAXD = 8
+FS_SU2_TASK_ROWS, FS_SU2_TASK_TABLE = 48, 1536
 
 # host tables passed by value with a launch
 FS_LIST_MAX = 96

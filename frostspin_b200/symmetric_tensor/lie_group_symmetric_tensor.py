@@ -643,6 +643,7 @@ class LieGroupSymmetricTensor(NonAbelianSymmetricTensor):
                 st["in_sb"], st["in_koff"], raw_s, st["out_sb"], st["out_moff"], ax)
             su2_fused_plan.check(fused[0], fused[1], int(self._data.numel()), out_size,
                                  int(st["u_host"].size))
+            su2_fused_plan.check_tasks(fused[0], fused[2])
             fused_coeffs = int((st["M"] * E)[fz].sum())
         if int(gather[0]["volume"].astype(np.int64).sum()) != x_size or int(
             scatter[0]["volume"].astype(np.int64).sum()

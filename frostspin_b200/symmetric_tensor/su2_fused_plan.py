@@ -15,11 +15,17 @@ indexes them (a test aid; the device path never calls it).
 
 import numpy as np
 
-from .._native import FS_PERM_MAXR, PERM_TASK_DTYPE, SU2_GROUP_DTYPE, SU2_PIECE_DTYPE
+from .._native import (
+    FS_PERM_MAXR,
+    FS_SU2_TASK_TABLE,
+    PERM_TASK_DTYPE,
+    SU2_GROUP_DTYPE,
+    SU2_PIECE_DTYPE,
+)
 from .abelian_plan import magic_divisor
 
 MAXD = 8
-TASK_TABLE = 1536   # FS_SU2_TASK_TABLE: (piece, row) offsets one task may hold
+TASK_TABLE = FS_SU2_TASK_TABLE   # (piece, row) offsets one task may hold
 TASK_ROWS = 768    # outer-leg values of a task of two pieces
 # Input coefficients of a task: enough to hide its descriptors behind the data
 # (TASK_COEFFS), fewer when the whole permute has less than one such task per
@@ -142,6 +148,33 @@ def check(gtab, pieces, src_len, out_len, u_len):
             raise AssertionError("fused permute piece rows outside the group")
         if not np.array_equal(np.bincount(gidx, weights=sr * sc, minlength=gtab.size), lim):
             raise AssertionError("fused permute pieces do not cover the group")
+
+
+def check_tasks(gtab, tasks):
+    """Every column of every group in exactly one task, and no task beyond the
+    offset table of the kernel, which skips such a task (host side check before the
+    call, like check())."""
+    g = tasks["eb"].astype(np.int64)
+    order = np.lexsort((tasks["start"], g))
+    g, start = g[order], tasks["start"][order].astype(np.int64)
+    end = start + tasks["count"][order]
+    ncols = gtab["ncols"].astype(np.int64)
+    first = np.concatenate([[True], g[1:] != g[:-1]]) if g.size else np.zeros(0, dtype=bool)
+    last = np.concatenate([first[1:], [True]]) if g.size else first
+    before = np.concatenate([[0], end[:-1]]) if g.size else end
+    if ((end <= start).any() or not np.array_equal(start, np.where(first, 0, before))
+            or not np.array_equal(end[last], ncols[g[last]])
+            or not np.array_equal(g[first], np.flatnonzero(ncols))):
+        raise AssertionError("fused permute tasks do not cover the columns")
+    # planes: values of the legs outside the two innermost
+    nd = gtab["ndim"].astype(np.int64)
+    d = gtab["dims"].astype(np.int64)
+    i = np.arange(gtab.size)
+    plane = (np.where(nd > 0, d[i, np.maximum(nd - 1, 0)], 1)
+             * np.where(nd > 1, d[i, np.maximum(nd - 2, 0)], 1))[g]
+    pieces = (gtab["in_count"].astype(np.int64) + gtab["out_count"])[g]
+    if (((end - 1) // plane - start // plane + 1) * pieces > FS_SU2_TASK_TABLE).any():
+        raise AssertionError("fused permute task beyond the kernel's offset table")
 
 
 def make_tasks(gtab):
