@@ -542,12 +542,13 @@ def _wide(arr):
     return int(a.max()) <= max_a
 
 
-# The tables cost the host about 100 us (318 recoupling products of an enlarged
-# corner, 141 us of device time: 1020 us a corner with them, 907 by value) and
-# are hidden only behind launches of milliseconds; there the per-tile kernel is
-# 0.6 % faster with them (10 335 tiles, 1.9e11 operations: 6.81 ms with tables,
-# 6.86 by value).  The streaming kernel is always faster by value (wide sectors
-# 313 us, with tables 336 us).
+# The tables cost the host about 100 us, and the device their copies and the launch
+# that expands the tiles; behind launches of milliseconds both are hidden, and the
+# per-tile kernel then runs a little faster with them.  Time by value over time with
+# tables, 23 launches of 2 to 350 sectors, equal and ragged, one transpose and all:
+# 3e9 FLOP 0.90-0.91, 1e10 0.98-0.99, 3e10 to 7e10 0.99-1.006, 1.2e11 to 1.8e12
+# 0.998-1.009, there above 1.003 in 20 of 26.  The streaming kernel is always faster by
+# value (wide sectors 313 us, with tables 336 us).
 _TABLE_FLOPS = 1e11
 
 
