@@ -7,18 +7,30 @@ import torch
 
 from frostspin_b200 import _native, linalg
 from frostspin_b200 import device as dev
+from frostspin_b200.symmetric_tensor import abelian_symmetric_tensor as ab
+from frostspin_b200.symmetric_tensor import lie_group_symmetric_tensor as lie
+from frostspin_b200.symmetric_tensor import o2_symmetric_tensor as o2
+
+
+def _clear_plans():
+    for cache in (ab._PLAN_CACHE, lie._MAP_CACHE, o2._PLAN_CACHE):
+        cache.clear()
 
 
 @pytest.fixture
 def launches(monkeypatch):
-    """The C ABI calls of host-memory tensors, recorded instead of made."""
+    """The C ABI calls of host-memory tensors, recorded instead of made.  The kernel's
+    limits are asked for before, and no plan with host tables outlives the test."""
     calls = []
+    lie._fused_limits()
+    _clear_plans()
     monkeypatch.setattr(dev, "device", lambda: torch.device("cpu"))
     monkeypatch.setattr(dev, "stream", lambda: 0)
     monkeypatch.setattr(dev, "upload", lambda a: torch.from_numpy(
         np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy()))
     monkeypatch.setattr(_native, "call", lambda name, *args, entry=None: calls.append((name, args)))
-    return calls
+    yield calls
+    _clear_plans()
 
 
 @pytest.mark.parametrize("n", [1, 200])   # tables by value and in device memory
@@ -136,15 +148,6 @@ def test_kept_tables_under_capture():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
-
-
-def _clear_plans():
-    from frostspin_b200.symmetric_tensor import abelian_symmetric_tensor as ab
-    from frostspin_b200.symmetric_tensor import lie_group_symmetric_tensor as lie
-    from frostspin_b200.symmetric_tensor import o2_symmetric_tensor as o2
-
-    for cache in (ab._PLAN_CACHE, lie._MAP_CACHE, o2._PLAN_CACHE):
-        cache.clear()
 
 
 @pytest.mark.gpu
