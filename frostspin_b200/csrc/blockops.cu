@@ -357,8 +357,8 @@ __global__ void __launch_bounds__(kOpThreads, 2)
                 for (int k = 0; k < kPerThread; ++k)
                     tile[wid + (k / 2) * kRowStep][lane + (k % 2) * 32] = vb[k];
                 __syncthreads();
-                // entries outside the block are zero in va only: B's zeros
-                // are placed at their own (c, r), inside the same mask
+                // entries outside the block are zero in va and in the tile, so a
+                // special value of either side meets only its own partner
 #pragma unroll
                 for (int k = 0; k < kPerThread; ++k)
                     part = fma(va[k], tile[lane + (k % 2) * 32][wid + (k / 2) * kRowStep], part);

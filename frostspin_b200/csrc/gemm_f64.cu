@@ -4,10 +4,12 @@
 //
 // Reference behaviour: SymmetricTensor.__matmul__ (frostspin/symmetric_tensor/
 // symmetric_tensor.py:453-489) calls numpy's dgemm once per shared irrep block.
-// Here every sector product of one contraction is a problem in one launch; the
-// host flattens all output tiles of all problems into a tile list and CTAs
-// stride over it (a static persistent schedule), so sectors of very uneven
-// sizes share the machine.
+// Here every sector product of one contraction is a problem in one launch, and
+// CTAs stride over the output tiles of all problems (a static persistent
+// schedule), so sectors of very uneven sizes share the machine.  Problems travel
+// with the kernel's parameters, and the CTAs enumerate the tiles themselves
+// (TileList); long lists and the longest launches read problems and tiles from
+// device memory (TileTable).
 //
 // 64x64 output tile per CTA, 4 warps of 32x32 (4x4 m8n8 fragments), k staged
 // 16 deep through a 3-stage cp.async pipeline, 3 CTAs per SM.  Sector blocks
@@ -449,7 +451,8 @@ extern "C" int fs_grouped_dgemm_uniform(const FsGemmProblem* d_problems, int64_t
 // through a small buffer into whole 64 NT-byte runs.  The 64 x 64 tiles of the
 // streaming kernel reload A for every tile by 8-byte cp.async and write C in
 // halves of sectors.  9 sectors with M = K = 7 to 51 and N = 0.1 to 0.2 M: 313 us
-// there (L2 write sectors 4 times the ideal), 201 us here.
+// there (L2 write sectors 4 times the ideal), 201 us here.  The 16 warps take 128
+// registers a thread; over all forms ptxas stores 132 and loads 508 spilled bytes.
 //
 // CTA b takes an equal share of the estimated time of all strips, problem by
 // problem, so it loads one or two A.  The host adds up the times: with every CTA

@@ -22,7 +22,8 @@
 // counts is warps in flight (40 per SM) rather than loads per warp.  The term
 // counts that occur (1 for reflections and copies, 2 for the merge, 4 for the
 // split) are separate forms with two columns per thread; the general loop over
-// up to four terms took 64 us for each cast of 5.6 M coefficients, this 55 us.
+// up to four terms took 64 us for each cast of 5.6 M coefficients, this 55 us,
+// with 80 bytes spilled at the 48 registers that ten CTAs per SM leave.
 // Tiles of 8 rows x 256 columns (100 registers) took 90 us; 32 x 32 tiles per
 // warp 48 us, but 17 us instead of 4.5 us at 70 000 coefficients.
 #include "common.cuh"

@@ -421,7 +421,7 @@ TILE_AREA = 128
 # and 10.5; 2.5 M 17.5 and 12.2; 4.5 M 29.6 and 17.8).
 TILE_TOTAL = 1_500_000
 MAX_TASK_TILES = 32   # kTileTaskMax
-TILE_TASKS = 4 * 3 * 148 * 4   # four tasks for every resident warp of the tile kernel
+TILE_TASKS = 3 * 148 * 4 * 4   # three tasks per resident warp (4 CTAs of 4 on each SM)
 
 
 def _make_tasks(ebs, chunk=TASK_CHUNK):
