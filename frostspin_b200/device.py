@@ -77,17 +77,17 @@ class KeptTables:
     def __init__(self):
         self._kept = None
 
-    def get(self, make):
-        """The tables of make() (nested tuples of tensors and None)."""
+    def get(self, make, s):
+        """The tables of make() (nested tuples of tensors and None), for launches on
+        the current stream s."""
         if self._kept is None:
             tables = make()
             if not torch.cuda.is_current_stream_capturing():
                 ready = torch.cuda.Event()
                 ready.record()
-                self._kept = (tables, ready, {stream()})
+                self._kept = (tables, ready, {s})
             return tables
         tables, ready, joined = self._kept
-        s = stream()
         if s not in joined and not torch.cuda.is_current_stream_capturing():
             current = torch.cuda.current_stream()
             current.wait_event(ready)

@@ -127,19 +127,20 @@ def upload_copies(tables):
     return dev.upload(ebs), dev.upload(tasks), dev.upload(tiles) if tiles.size else None
 
 
-def run_copies(tables, device_tables, src, out):
-    """One batch of strided copies src -> out: the row tasks in one launch, the
-    transposed ones, if any, in another."""
+def run_copies(tables, device_tables, src, out, stream=None):
+    """One batch of strided copies src -> out on the current stream (`stream`, if the
+    caller has asked for it already): the row tasks in one launch, the transposed ones,
+    if any, in another."""
+    if stream is None:
+        stream = dev.stream()
     ebs, tasks, tiles = tables
     d_ebs, d_tasks, d_tiles = device_tables
     if tasks.size or d_tiles is None:
         _native.call("fs_abelian_permute", dev.ptr(src), src.numel(), dev.ptr(out), out.numel(),
-                     d_ebs.data_ptr(), ebs.size, d_tasks.data_ptr(), tasks.size, None,
-                     dev.stream())
+                     d_ebs.data_ptr(), ebs.size, d_tasks.data_ptr(), tasks.size, None, stream)
     if d_tiles is not None:
         _native.call("fs_permute_tiles", dev.ptr(src), src.numel(), dev.ptr(out), out.numel(),
-                     d_ebs.data_ptr(), ebs.size, d_tiles.data_ptr(), tiles.size, None,
-                     dev.stream())
+                     d_ebs.data_ptr(), ebs.size, d_tiles.data_ptr(), tiles.size, None, stream)
 
 
 def defer_permute(tables, src, out, nbytes):

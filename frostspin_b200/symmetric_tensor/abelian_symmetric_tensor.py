@@ -187,7 +187,8 @@ class AbelianSymmetricTensor(SymmetricTensor):
         if plan.size and linalg.defer_permute(tables, self._data, out, 16.0 * plan.size):
             return out, plan.offsets, plan.block_shapes, plan.block_irreps
         if plan.size:
-            d_tables = plan.device_tables.get(lambda: linalg.upload_copies(tables))
+            s = dev.stream()
+            d_tables = plan.device_tables.get(lambda: linalg.upload_copies(tables), s)
             with instrument.region("permute", bytes=16.0 * plan.size):
-                linalg.run_copies(tables, d_tables, self._data, out)
+                linalg.run_copies(tables, d_tables, self._data, out, s)
         return out, plan.offsets, plan.block_shapes, plan.block_irreps

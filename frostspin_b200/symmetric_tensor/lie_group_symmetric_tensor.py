@@ -171,7 +171,8 @@ class LieMap:
         )
 
     def run(self, src, out=None):
-        d_gather, d_scatter, d_u, d_fz = self.device.get(self._upload)
+        stream = dev.stream()
+        d_gather, d_scatter, d_u, d_fz = self.device.get(self._upload, stream)
         if out is None:
             out = dev.zeros_f64(self.out_size) if self.zero_out else dev.empty_f64(self.out_size)
         if src.numel() < self.in_len:
@@ -184,14 +185,14 @@ class LieMap:
                     int(out.numel()), d_groups.data_ptr(), int(self.fused[0].size),
                     d_pieces.data_ptr(), int(self.fused[1].size), d_u.data_ptr(),
                     int(self.u_host.size), d_tasks.data_ptr(), int(self.fused[2].size), None,
-                    dev.stream(),
+                    stream,
                 )
         if self.x_size == 0:
             return out
         x = dev.empty_f64(self.x_size)
         y = dev.empty_f64(int((self.M * self.N).sum()))
         with instrument.region("permute", bytes=16.0 * self.x_size):
-            linalg.run_copies(self.gather, d_gather, src, x)
+            linalg.run_copies(self.gather, d_gather, src, x, stream)
         arr = np.zeros(self.M.size, dtype=_native.GEMM_PROBLEM_DTYPE)
         y_off = _exclusive_cumsum(self.M * self.N)
         arr["A"] = d_u.data_ptr() + 8 * self.u_off
@@ -204,7 +205,7 @@ class LieMap:
         arr["alpha"] = 1.0
         linalg.grouped_dgemm_table(arr, region="gemm_recoupling")
         with instrument.region("permute", bytes=16.0 * int(y.numel())):
-            linalg.run_copies(self.scatter, d_scatter, y, out)
+            linalg.run_copies(self.scatter, d_scatter, y, out, stream)
         return out
 
 

@@ -272,15 +272,17 @@ class _Recombine:
         out = dev.empty_f64(self.out_len)
         if self.blocks.size == 0 or self.out_len == 0:
             return out
+        stream = dev.stream()
         d_blocks, d_index, d_coef = self.device_tables.get(
-            lambda: (dev.upload(self.blocks), dev.upload(self.index), dev.upload(self.coef)))
+            lambda: (dev.upload(self.blocks), dev.upload(self.index), dev.upload(self.coef)),
+            stream)
         with instrument.region("o2_recombine", bytes=16.0 * self.out_len):
             for start in range(0, self.blocks.size, _MAX_BLOCKS_PER_CALL):
                 cnt = min(_MAX_BLOCKS_PER_CALL, self.blocks.size - start)
                 _native.call(
                     "fs_o2_recombine", dev.ptr(src), int(src.numel()), dev.ptr(out),
                     self.out_len, d_blocks.data_ptr() + start * self.blocks.itemsize, cnt,
-                    d_index.data_ptr(), d_coef.data_ptr(), self.max_rows, None, dev.stream(),
+                    d_index.data_ptr(), d_coef.data_ptr(), self.max_rows, None, stream,
                 )
         return out
 
