@@ -338,7 +338,9 @@ def grouped_dgemm_table(arr, region="gemm_fp64"):
 # rates of the two paths on B200 inside the SU(2) CTMRG workload (int8: the
 # CTA-pair k_oz_gemm_pair; FP64: k_grouped_dgemm averaged over the sector
 # shapes it receives), used only to decide which path a sector GEMM takes in a
-# mixed-precision run
+# mixed-precision run that is not tuned.  They are the rates before the wide kernel
+# (up to 25 TF/s) and the present split (5.4 TB/s); those would move sectors both
+# ways, and untuned runs keep the arithmetic that they had.
 _INT8_OPS = 1.8e15
 _FP64_FLOPS = 2.0e13
 _EPILOGUE_BPS = 2.0e12
