@@ -350,7 +350,8 @@ def check(status, what):
 # timed region from these counters)
 CALL_COUNTS = {}
 
-# kernels each entry point launches
+# kernels each entry point launches, at least (fs_diag_mul: a second one for thin
+# transposed blocks)
 LAUNCHES_PER_CALL = {
     "fs_abelian_permute": 1, "fs_abelian_permute_multi": 1,
     "fs_permute_tiles": 1, "fs_permute_tiles_multi": 1, "fs_su2_permute_fused": 1, "fs_grouped_dgemm": 1, "fs_grouped_dgemm_thin": 1,
