@@ -231,9 +231,16 @@ def grouped_gemm(problems):
     run_gemm_table(arr, problems)
 
 
+_MAX_SIDE = 2**31 - 1   # FsGemmProblem M, N, K
+
+
 def block_gemm(a, a_off, a_trans, b, b_off, b_trans, c, c_off, M, N, K):
     """C_i = op(A_i) op(B_i) for blocks of three buffers: element offsets and
     sizes as int64 arrays, C-order results, one launch (see grouped_gemm)."""
+    # no side is longer than a buffer that holds a block of it; assigned arrays wrap
+    if (max(a.numel(), b.numel(), c.numel()) > _MAX_SIDE
+            and max(int(x.max(initial=0)) for x in (M, N, K)) > _MAX_SIDE):
+        raise OverflowError("a block side exceeds the 32 bits of a GEMM problem")
     arr = np.zeros(len(M), dtype=_native.GEMM_PROBLEM_DTYPE)
     arr["A"] = a.data_ptr() + 8 * a_off
     arr["B"] = b.data_ptr() + 8 * b_off
