@@ -915,7 +915,8 @@ def weighted_reduce(buf, offsets, lengths, weights, *, squares):
     """sum_s w_s sum_i f(buf[off_s + i]) with f = x^2 or x; returns a 0-d device
     tensor (no host synchronisation)."""
     sums = dev.reduction_buffer(buf.device)
-    out, part, n_part = sums[0], sums.data_ptr() + 8, sums.numel() - 1
+    out, n_part = sums.data_ptr(), sums.numel() - 1
+    part = out + 8
     segs = np.zeros(len(offsets), dtype=_native.SEGMENT_DTYPE)
     segs["offset"] = offsets
     segs["length"] = lengths
@@ -923,9 +924,9 @@ def weighted_reduce(buf, offsets, lengths, weights, *, squares):
     name = "fs_weighted_sumsq" if squares else "fs_weighted_sum"
     if segs.size <= _native.FS_LIST_MAX:
         _native.call(name, dev.ptr(buf), segs.ctypes.data, segs.size, int(squares),
-                     part, n_part, out.data_ptr(), dev.stream(),
+                     part, n_part, out, dev.stream(),
                      entry="fs_weighted_sum_list")
-        return out
+        return sums[0]
     d_segs = dev.upload(segs)
     _native.call(
         name,
@@ -934,26 +935,27 @@ def weighted_reduce(buf, offsets, lengths, weights, *, squares):
         segs.size,
         part,
         n_part,
-        out.data_ptr(),
+        out,
         dev.stream(),
     )
-    return out
+    return sums[0]
 
 
 def pair_contract(abuf, bbuf, pairs):
     """pairs: list of (a_off, b_off, m, n, a_trans, b_trans, weight); b_off < 0
     means trace of the A block.  Returns a 0-d device tensor."""
-    sums = dev.reduction_buffer(abuf.device)
-    out, part, n_part = sums[0], sums.data_ptr() + 8, sums.numel() - 1
+    sums = dev.reduction_buffer(abuf.device)   # its view is made behind the launch
+    out, n_part = sums.data_ptr(), sums.numel() - 1
+    part = out + 8
     tab = np.zeros(len(pairs), dtype=_native.PAIR_BLOCK_DTYPE)
     if len(pairs):
         tab[:] = [tuple(p) for p in pairs]
     b_ptr = dev.ptr(bbuf) if bbuf is not None else None
     if tab.size <= _native.FS_LIST_MAX:
         _native.call("fs_pair_contract", dev.ptr(abuf), b_ptr, tab.ctypes.data, tab.size,
-                     part, n_part, out.data_ptr(), dev.stream(),
+                     part, n_part, out, dev.stream(),
                      entry="fs_pair_contract_list")
-        return out
+        return sums[0]
     d_tab = dev.upload(tab)
     _native.call(
         "fs_pair_contract",
@@ -963,10 +965,10 @@ def pair_contract(abuf, bbuf, pairs):
         tab.size,
         part,
         n_part,
-        out.data_ptr(),
+        out,
         dev.stream(),
     )
-    return out
+    return sums[0]
 
 
 def axpby(x, y, a, b):
